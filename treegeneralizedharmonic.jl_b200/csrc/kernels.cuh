@@ -35,8 +35,11 @@ struct HookPt {
 };
 
 // A block's working array per variable is Wd^3 points (the reference's ghosted cube) stored
-// with rows of Wx >= Wd doubles (Wx even: every row starts on a 16-byte boundary, as the tensor
-// copies into shared memory require); point (x, y, z) of the cube sits at x + Wx (y + Wd z).
+// with rows of Wx >= Wd doubles (row_pitch); point (x, y, z) of the cube sits at x + Wx (y + Wd z).
+// The array starts XO = row_lead doubles into its allocation, so that every row's owned points
+// (x >= G) start on a 32-byte sector: a warp on consecutive owned points touches whole sectors,
+// pairs of points from an even one are one 16-byte load, and the tensor copies into shared
+// memory start on the 16 bytes they need.
 struct Geo {
   int N1, Wd, G, Wx;
   long S, Wv;  // points per block in state layout; doubles per block and variable in work layout

@@ -43,6 +43,14 @@ namespace tgh {
 constexpr int NC = 10;
 constexpr int NV = 20;
 
+// Row layout of the device arrays, in doubles (a 32-byte sector is 4): a working array's rows of
+// Wd points have the pitch row_pitch and start row_lead doubles into the allocation, which puts
+// the first owned point (G points in) on a sector; arrays held per computed point have rows of
+// N1 points at point_pitch.
+TGH_HD constexpr int row_lead(int G) { return (4 - G % 4) % 4; }
+TGH_HD constexpr int row_pitch(int Wd, int G) { return (Wd + row_lead(G) + 3) / 4 * 4; }
+TGH_HD constexpr int point_pitch(int N1) { return (N1 + 3) / 4 * 4; }
+
 // packed slot of the symmetric pair (a, b), 0-based, column-major lower triangle
 TGH_HD constexpr int pidx(int a, int b) {
   return (a > b ? b : a) * 4 - ((a > b ? b : a) * ((a > b ? b : a) - 1)) / 2 + ((a > b ? a : b) - (a > b ? b : a));

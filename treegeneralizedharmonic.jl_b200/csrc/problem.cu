@@ -24,9 +24,9 @@
 using namespace tgh;
 
 namespace tgh {
-bool make_pi_tma_maps(double* work, int nwb, PiTmaMaps* out, std::string& err);
-cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const Case& cs, const RhsArgs& a, const PiTmaMaps& M,
-                          PiTmaStatus st, int b0, int nb);
+bool make_tma_maps(double* work, int nwb, TmaMaps* out, std::string& err);
+cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
+                          int b0, int nb);
 }  // namespace tgh
 
 // the Pi kernel a problem launches: the one-point kernel reading through L1, or the pair kernel
@@ -53,6 +53,7 @@ struct tgh_problem {
   // nb: the blocks this rank computes (its own leaves); nwb: the working arrays' blocks, its
   // own leaves first, then the halo: other ranks' leaves its fill reads
   int q, G, N, N1, Wd, Wx, nb, nwb, maxlevel = 0;  // Wx: the working array's row pitch
+  int XO = 0;  // doubles ahead of a row's first point, so that its owned points start on a sector (row_lead)
   double lo[3], h0;
   int cells0[3], periodic[3];
   std::vector<int> level, corner;  // of every leaf of the forest (global numbering)
@@ -62,7 +63,9 @@ struct tgh_problem {
   std::vector<ExchangeList> xch;   // per fill phase: 0 the copies, l >= 1 level l's prolongation
   std::vector<std::unordered_map<int64_t, int>> lut;
   Geo geo;
+  int NX = 0;   // the coefficients' and the accumulator's row pitch (point_pitch)
   long S, Wv, npts;
+  long SX = 0;  // NX N1^2: their doubles per block and variable
   Case cs;
   bool diss = false, intr = false;
   bool mixed = false;  // TGH_PREC_MIXED: FP32 stencil sums and algebra, FP64 state and metric
@@ -145,7 +148,7 @@ struct tgh_problem {
   int pi_variant = PI_L1;
   int threads = 128;  // CTA size of the head and one-point Pi kernels
   int pi_mb = 4;      // the one-point Pi kernel's resident CTAs per SM (its launch bound)
-  std::vector<std::pair<const double*, PiTmaMaps>> tma_maps;
+  std::vector<std::pair<const double*, TmaMaps>> tma_maps;
   int* dev_err = nullptr;                 // a bounded device wait that gave up records it here
   // the blocks interior_kernel visits: those that can hold a point with r < r_1 at some time of
   // [lo, hi]; one list for direct launches, one for the captured graph (built before capture)
@@ -177,8 +180,19 @@ static int fail(tgh_problem* p, int code, const std::string& msg) {
   return code;
 }
 
-// doubles in one of the problem's working arrays (rows padded to the pitch Wx)
+// doubles in one of the problem's working arrays (rows padded to the pitch Wx), and in the
+// arrays held per computed point (the accumulator; rows padded to the pitch NX)
 static size_t work_doubles(const tgh_problem* p) { return (size_t)p->Wv * NV * p->nwb; }
+static size_t acc_doubles(const tgh_problem* p) { return (size_t)p->SX * NV * p->nb; }
+// a working array, zeroed; freed at (pointer - XO)
+static cudaError_t alloc_work(tgh_problem* p, double** out) {
+  const size_t bytes = (work_doubles(p) + p->XO) * sizeof(double);
+  double* base = nullptr;
+  cudaError_t e = cudaMalloc(&base, bytes);
+  if (e != cudaSuccess) return e;
+  *out = base + p->XO;
+  return cudaMemsetAsync(base, 0, bytes, p->stream);
+}
 // a padded work index as the index of the same point in the reference's dense cube
 static int dense_index(const tgh_problem* p, int w) { return (w % p->Wx) + p->Wd * (w / p->Wx); }
 
@@ -739,17 +753,17 @@ static cudaError_t launch_part(tgh_problem* p, int part, int mode, cudaStream_t 
 }
 
 // whether a launch may take the TMA Pi kernel: the variant chosen, its configuration, whole blocks
-static bool pi_tma_applies(const tgh_problem* p, const RhsArgs& a) {
+static bool tma_applies(const tgh_problem* p, const RhsArgs& a) {
   return p->pi_variant == PI_TMA && p->q == 4 && p->N == 32 && !p->mixed && a.p0 % p->S == 0 && a.p1 % p->S == 0;
 }
 
 // the tensor maps of one of the problem's working arrays (made once per array)
-static const PiTmaMaps* pi_tma_maps(tgh_problem* p, const double* work) {
+static const TmaMaps* work_tma_maps(tgh_problem* p, const double* work) {
   for (auto& e : p->tma_maps)
     if (e.first == work) return &e.second;
-  PiTmaMaps m;
+  TmaMaps m;
   std::string err;
-  if (!make_pi_tma_maps(const_cast<double*>(work), p->nwb, &m, err)) {
+  if (!make_tma_maps(const_cast<double*>(work) - p->XO, p->nwb, &m, err)) {
     p->err = err;
     return nullptr;
   }
@@ -828,11 +842,11 @@ static int launch_rhs(tgh_problem* p, const RhsArgs& a, int mode) {
     if (s) return s;
   }
   CK(launch_part(p, 0, mode, p->stream, a));
-  if (pi_tma_applies(p, a)) {
-    const PiTmaMaps* M = pi_tma_maps(p, a.work);
+  if (tma_applies(p, a)) {
+    const TmaMaps* M = work_tma_maps(p, a.work);
     if (!M) return TGH_ERR_CUDA;
-    CK(launch_pi_tma(p->diss, mode, p->stream, p->cs, a, *M, PiTmaStatus{p->dev_err, p->wait_limit},
-                     (int)(a.p0 / p->S), (int)((a.p1 - a.p0) / p->S)));
+    CK(launch_pi_tma(p->diss, mode, p->stream, a, *M, WaitStatus{p->dev_err, p->wait_limit}, (int)(a.p0 / p->S),
+                     (int)((a.p1 - a.p0) / p->S)));
     return TGH_OK;
   }
   CK(launch_part(p, 1, mode, p->stream, a));
@@ -850,6 +864,8 @@ static RhsArgs base_args(tgh_problem* p, const double* work, double t) {
   a.Wd = p->Wd;
   a.Wx = p->Wx;
   a.G = p->G;
+  a.NX = p->NX;
+  a.ncoef = p->SX * p->nb;
   a.npts = p->npts;
   a.p0 = 0;
   a.p1 = p->npts;
@@ -988,7 +1004,9 @@ static int setup_host(tgh_problem* p, const tgh_config* cfg, const tgh_mesh* m, 
   p->N = m->N;
   p->N1 = m->N + 1;
   p->Wd = m->N + 2 * p->G + 1;
-  p->Wx = p->Wd + (p->Wd & 1);
+  p->XO = row_lead(p->G);
+  p->Wx = row_pitch(p->Wd, p->G);
+  p->NX = point_pitch(p->N1);
   p->h0 = m->h0;
   for (int d = 0; d < 3; ++d) {
     p->lo[d] = m->lo[d];
@@ -1011,6 +1029,7 @@ static int setup_host(tgh_problem* p, const tgh_config* cfg, const tgh_mesh* m, 
   }
   p->S = (long)p->N1 * p->N1 * p->N1;
   p->Wv = (long)p->Wx * p->Wd * p->Wd;
+  p->SX = (long)p->NX * p->N1 * p->N1;
   p->npts = p->S * p->nb;
   p->geo = Geo{p->N1, p->Wd, p->G, p->Wx, p->S, p->Wv};
   if (cfg->bg.kind < TGH_BG_MINKOWSKI || cfg->bg.kind > TGH_BG_HARMONIC_KERR)
@@ -1071,13 +1090,12 @@ static int setup_device(tgh_problem* p) {
   }
   CK(cudaMalloc(&p->blk, blk.size() * sizeof(double)));
   CK(cudaMemcpy(p->blk, blk.data(), blk.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&p->work, (size_t)p->Wv * NV * p->nwb * sizeof(double)));
-  CK(cudaMemsetAsync(p->work, 0, (size_t)p->Wv * NV * p->nwb * sizeof(double), p->stream));
+  CK(alloc_work(p, &p->work));
   CK(cudaMalloc(&p->scratch, 2 * sizeof(unsigned long long)));
   CK(cudaMalloc(&p->bcounts, 3 * sizeof(unsigned long long)));
   CK(cudaMalloc(&p->dev_err, sizeof(int)));
   CK(cudaMemsetAsync(p->dev_err, 0, sizeof(int), p->stream));
-  CK(cudaMalloc(&p->coef, (size_t)NCOEF * p->npts * sizeof(double)));
+  CK(cudaMalloc(&p->coef, (size_t)NCOEF * p->SX * p->nb * sizeof(double)));
   p->npart = (int)grid_for(p->npts, 128);
   CK(cudaMalloc(&p->part, (3 * (size_t)p->npart + 2) * sizeof(double)));
   CK(cudaMalloc(&p->diag, (size_t)NDIAG * p->npts * sizeof(double)));
@@ -1127,10 +1145,12 @@ void tgh_problem_destroy(tgh_problem* p) {
     if (x.send) cudaFree(x.send);
     if (x.recv) cudaFree(x.recv);
   }
-  void* bufs[] = {p->work, p->Hsrc, p->tw, p->tf, p->blk, p->primary, p->runs, p->gpts, p->hooks, p->hook_cache, p->scratch,
+  for (double* w : {p->work, p->W1, p->W2, p->twork})
+    if (w) cudaFree(w - p->XO);
+  void* bufs[] = {p->Hsrc, p->tw, p->tf, p->blk, p->primary, p->runs, p->gpts, p->hooks, p->hook_cache, p->scratch,
                   p->bcounts, p->dev_err, p->ilist.dev, p->ilist_graph.dev,
                   p->part, p->coef, p->diag, p->dpart, p->ind, p->ind_tol, p->ind_counts, p->ind_boxes,
-                  p->k, p->acc, p->y, p->u0, p->W1, p->W2, p->bacc, p->twork, p->kt, p->acct, p->yt,
+                  p->k, p->acc, p->y, p->u0, p->bacc, p->kt, p->acct, p->yt,
                   p->adj_cot, p->adj_mu, p->adj_part, p->adj_y[0], p->adj_y[1], p->adj_y[2], p->adj_a,
                   p->adj_acc, p->adj_m};
   for (void* b : bufs)
@@ -1428,7 +1448,7 @@ int tgh_set_variant(tgh_problem* p, int pi_variant, int threads, int pi_mb) {
   if (pi_mb < 3 || pi_mb > 5) return fail(p, TGH_ERR_ARG, "the one-point Pi kernel's CTAs per SM must be 3, 4 or 5");
   if (pi_variant == TGH_PI_TMA) {
     // check now that the driver can describe the working array to the copy engine
-    if (!pi_tma_maps(p, p->work)) return TGH_ERR_CUDA;
+    if (!work_tma_maps(p, p->work)) return TGH_ERR_CUDA;
   }
   p->pi_variant = pi_variant;
   p->threads = threads;
@@ -1803,12 +1823,10 @@ static int launch_fill_phase(tgh_problem* p, double* work, int phase, double t) 
 
 static int batched_buffers(tgh_problem* p) {
   if (p->W1) return TGH_OK;
-  const size_t Lw = work_doubles(p), L = tgh_state_length(p);
-  CK(cudaMalloc(&p->W1, Lw * sizeof(double)));
-  CK(cudaMalloc(&p->W2, Lw * sizeof(double)));
-  CK(cudaMalloc(&p->bacc, L * sizeof(double)));
-  CK(cudaMemsetAsync(p->W1, 0, Lw * sizeof(double), p->stream));
-  CK(cudaMemsetAsync(p->W2, 0, Lw * sizeof(double), p->stream));
+  CK(alloc_work(p, &p->W1));
+  CK(alloc_work(p, &p->W2));
+  CK(cudaMalloc(&p->bacc, acc_doubles(p) * sizeof(double)));
+  CK(cudaMemsetAsync(p->bacc, 0, acc_doubles(p) * sizeof(double), p->stream));
   return TGH_OK;
 }
 
@@ -2053,14 +2071,10 @@ int tgh_shard_end(tgh_problem* p, double* u) {
 // events on the problem's stream over nlaunch launches. mode 0: the plain form's kernel
 // (du); mode 1: the batched form's kernel with the stage-2 epilogue. u is filled first.
 int tgh_time_rhs(tgh_problem* p, const double* u, double t, int mode, int nlaunch, double* ms_per_launch) {
-  const size_t L = tgh_state_length(p), Lw = work_doubles(p);
+  const size_t L = tgh_state_length(p);
   if (mode == 0 && !p->k) CK(cudaMalloc(&p->k, L * sizeof(double)));
-  if (mode == 1 && !p->W1) {
-    CK(cudaMalloc(&p->W1, Lw * sizeof(double)));
-    CK(cudaMalloc(&p->W2, Lw * sizeof(double)));
-    CK(cudaMalloc(&p->bacc, L * sizeof(double)));
-    CK(cudaMemsetAsync(p->bacc, 0, L * sizeof(double), p->stream));
-  }
+  if (mode == 1)
+    if (int st = batched_buffers(p)) return st;
   // a rank of a sharded problem cannot fill from u alone: it is timed on its working array as
   // its last step left it (filled)
   int s = p->nranks > 1 ? TGH_OK : prepare_impl(p, u, t, "tgh_time_rhs");
@@ -2128,11 +2142,8 @@ static int tangent_check(tgh_problem* p, int dir) {
   if (p->mixed) return fail(p, TGH_ERR_ARG, "the tangent-linear form is FP64");
   if (p->intr && (core_follows(p->cs) || p->cfg.interior == TGH_INT_PASTED || p->cfg.interior == TGH_INT_FITTED))
     return fail(p, TGH_ERR_ARG, "the tangent-linear form takes a static :damped or :frozen interior");
-  const size_t L = tgh_state_length(p), Lw = work_doubles(p);
-  if (!p->twork) {
-    CK(cudaMalloc(&p->twork, Lw * sizeof(double)));
-    CK(cudaMemsetAsync(p->twork, 0, Lw * sizeof(double), p->stream));
-  }
+  const size_t L = tgh_state_length(p);
+  if (!p->twork) CK(alloc_work(p, &p->twork));
   if (!p->kt) {
     CK(cudaMalloc(&p->kt, L * sizeof(double)));
     CK(cudaMalloc(&p->acct, L * sizeof(double)));

@@ -181,8 +181,8 @@ template <int Q, class T> __device__ __forceinline__ T st_mixed(const double* p,
   return acc;
 }
 
-// Per-point coefficients the head kernel leaves for the Pi kernel (struct of arrays,
-// slot c of point p at coef[c * npts + p]).
+// Per-point coefficients the head kernel leaves for the Pi kernel (struct of arrays, slot c of a
+// point at coef[c * ncoef + PointIdx::cp]: rows of N1 points, NX apart, so that they start on a sector).
 enum {
   CF_B0 = 0, CF_B1, CF_B2,            // beta^i
   CF_DIVB,                            // d_i beta^i
@@ -201,15 +201,17 @@ struct RhsArgs {
   const double* Hsrc;     // sampled gauge source, (N1^3 x 20) per block, or null
   const double* matter;   // (N1^3 x 10) per block, or null
   const double* blk;      // per block: domain lo (3), h, integer corner (3), pad
-  double* coef;           // NCOEF x npts scratch between the two kernels
+  double* coef;           // NCOEF x ncoef scratch between the two kernels (rows of N1 points NX apart)
   double* du;             // MODE_DU: state layout
   // MODE_STAGE
   const double* u0;       // state at the start of the step (ghosted layout)
-  double* acc;            // accumulator (state layout)
+  double* acc;            // accumulator (state layout with rows NX apart)
   double* next;           // the next stage's ghosted working array (owned points written)
   double ca, cb;          // next = u0 + ca k ; acc = (stage 1 ? u0 : acc) + cb k ; final: next = acc + cb k
   int stage;              // 1..4
   int N1, Wd, G, Wx;      // block edge + 1, ghosted cube edge, ghost width, row pitch
+  int NX;                 // row pitch of the coefficients and the accumulator
+  long ncoef;             // doubles per coefficient slot: NX N1^2 * nblocks
   long npts;              // N1^3 * nblocks
   long p0, p1;            // the points [p0, p1) this launch covers (whole blocks)
   double t;
@@ -228,7 +230,7 @@ struct EmitStage {
   double* ac;
   double* nx;
   const double* u0;
-  long S, sv;
+  long S, sv;  // per variable: of the accumulator, of the working array
   double ca, cb;
   int stage;
   __device__ __forceinline__ void put(int v, double kv) {
@@ -256,7 +258,8 @@ struct EmitStage {
 // the owned point p of a launch: block, index within the block, position, work offset
 struct PointIdx {
   int b, i, j, k;
-  long ip, wo;
+  long ip, wo;   // the point in a block of the state layout, and in the working array
+  long cp, ap;   // in a coefficient slot, and in the accumulator
   double x[3], h;
 };
 __device__ __forceinline__ PointIdx point_index(const RhsArgs& A, long p) {
@@ -275,6 +278,10 @@ __device__ __forceinline__ PointIdx point_index(const RhsArgs& A, long p) {
   q.x[2] = __dadd_rn(bl[2], __dmul_rn(bl[6] + (double)q.k, q.h));
   const long sv = (long)A.Wx * A.Wd * A.Wd;
   q.wo = (long)q.b * NV * sv + (q.i + A.G) + (long)A.Wx * ((q.j + A.G) + (long)A.Wd * (q.k + A.G));
+  const long SX = (long)A.NX * N1 * N1;
+  const long ic = q.i + (long)A.NX * (q.j + (long)N1 * q.k);
+  q.cp = (long)q.b * SX + ic;
+  q.ap = (long)q.b * NV * SX + ic;
   return q;
 }
 
@@ -286,7 +293,8 @@ template <int Q, int N1S> __device__ __forceinline__ RhsArgs fixed_geometry(cons
     B.N1 = N1S;
     B.G = Q / 2 + 1;
     B.Wd = N1S + 2 * (Q / 2 + 1);
-    B.Wx = B.Wd + (B.Wd & 1);
+    B.Wx = row_pitch(B.Wd, B.G);
+    B.NX = point_pitch(N1S);
   }
   return B;
 }
@@ -389,7 +397,7 @@ __device__ __forceinline__ void store_matter(const Coef<T>& C, const RhsArgs& A,
   for (int k = 0; k < 10; ++k) m[k] = ldk<T>(q + k * S);
   matter_source(C, m, ms);
 #pragma unroll
-  for (int v = 0; v < NC; ++v) cfo[(CF_M0 + v) * A.npts] = value(ms[v]);
+  for (int v = 0; v < NC; ++v) cfo[(CF_M0 + v) * A.ncoef] = value(ms[v]);
 }
 
 // Step 3 (src/evolution.jl:286-297): the gauge source (sampled, closed-form Kerr-Schild or
@@ -475,9 +483,10 @@ __global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsA
   if (r >= cs.r1) return;
   const long sv = (long)A.Wx * A.Wd * A.Wd;
   const double* wk = A.work + q.wo;
-  double* cfo = A.coef + p;
+  double* cfo = A.coef + q.cp;
+  const long SX = (long)A.NX * A.N1 * A.N1;
   EmitDu ed{A.du + (long)q.b * NV * S + q.ip, S};
-  EmitStage es{A.acc + (long)q.b * NV * S + q.ip, A.next + q.wo, A.u0 + q.wo, S, sv, A.ca, A.cb, A.stage};
+  EmitStage es{A.acc + q.ap, A.next + q.wo, A.u0 + q.wo, SX, sv, A.ca, A.cb, A.stage};
   auto put = [&](int v, double val) {
     if (MODE == MODE_DU) ed.put(v, val);
     else es.put(v, val);
@@ -501,9 +510,9 @@ __global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsA
     double w, rho;
     layer_profiles(cs, r, w, rho);
     const double om = 1.0 - w;
-    double* dD = MODE == MODE_DU ? ed.d : cfo + CF_DTH0 * A.npts;
+    double* dD = MODE == MODE_DU ? ed.d : cfo + CF_DTH0 * A.ncoef;
     double* dT = MODE == MODE_DU ? ed.d + NC * S : es.nx + NC * sv;
-    const long sD = MODE == MODE_DU ? S : A.npts, sT = MODE == MODE_DU ? S : sv;
+    const long sD = MODE == MODE_DU ? S : A.ncoef, sT = MODE == MODE_DU ? S : sv;
     for (int v = 0; v < NV; ++v) {
       const double sl = tw[(NV + v) * S];
       const double tg = tw[v * S] + dt * sl;
@@ -521,7 +530,7 @@ __global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsA
     if (MODE == MODE_DU)
       layer_targets(cs, A.t, q.x, wk, sv, w, rho, ed.d, S, ed.d + NC * S, S);
     else
-      layer_targets(cs, A.t, q.x, wk, sv, w, rho, cfo + CF_DTH0 * A.npts, A.npts, es.nx + NC * sv, sv);
+      layer_targets(cs, A.t, q.x, wk, sv, w, rho, cfo + CF_DTH0 * A.ncoef, A.ncoef, es.nx + NC * sv, sv);
     return;
   }
   if (!core_follows(cs)) {
@@ -578,14 +587,15 @@ __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(con
   const long sv = (long)A.Wx * A.Wd * A.Wd;
   const double* wk = A.work + q.wo;
   const double inv_h = 1.0 / q.h;
-  double* cfo = A.coef + p;
+  double* cfo = A.coef + q.cp;
+  const long SX = (long)A.NX * A.N1 * A.N1;
   EmitDu ed{A.du + (long)q.b * NV * S + q.ip, S};
-  EmitStage es{A.acc + (long)q.b * NV * S + q.ip, A.next + q.wo, A.u0 + q.wo, S, sv, A.ca, A.cb, A.stage};
+  EmitStage es{A.acc + q.ap, A.next + q.wo, A.u0 + q.wo, SX, sv, A.ca, A.cb, A.stage};
   // d_t h of an evolved point: stored at once in the plain form; in the batched form parked in
   // the coefficients, and the Pi kernel (more warps to cover the loads) does its stage update
   auto put_dth = [&](int v, double val) {
     if (MODE == MODE_DU) ed.put(v, val);
-    else cfo[(CF_DTH0 + v) * A.npts] = val;
+    else cfo[(CF_DTH0 + v) * A.ncoef] = val;
   };
   double w = 1.0, rho = 0.0, r = 0.0;
   if (INT) {
@@ -594,7 +604,7 @@ __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(con
     r = interior_radius(cs, A.t, q.x);
     const bool frozen = cs.interior == TGH_INT_PASTED ? r < cs.r1 : r < cs.r0;
     if (frozen) {
-      cfo[CF_W * A.npts] = -1.0;
+      cfo[CF_W * A.ncoef] = -1.0;
       return;
     }
     if (r < cs.r1) layer_profiles(cs, r, w, rho);
@@ -611,15 +621,15 @@ __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(con
     for (int v = 0; v < NC; ++v) put_dth(v, (double)dth[v]);
   } else {
     // w d_t h + D, D parked at the layer's entry in the slot this value replaces
-    const double* dD = MODE == MODE_DU ? ed.d : cfo + CF_DTH0 * A.npts;
-    const long sD = MODE == MODE_DU ? S : A.npts;
+    const double* dD = MODE == MODE_DU ? ed.d : cfo + CF_DTH0 * A.ncoef;
+    const long sD = MODE == MODE_DU ? S : A.ncoef;
 #pragma unroll
     for (int v = 0; v < NC; ++v) put_dth(v, fma(w, (double)dth[v], dD[v * sD]));
   }
   // the Pi coefficients (and the matter term), then the source, in the form's arithmetic
   const T* dh[3] = {dh0, dh1, dh2};
   const Coef<T> Ct = coef_in<T>(C);
-  store_pi_coefficients(Ct, dh, eh, cfo, A.npts);
+  store_pi_coefficients(Ct, dh, eh, cfo, A.ncoef);
   if (A.matter) store_matter(Ct, A, q.b, q.ip, cfo);
   T msrc[NC], ht[NC];
 #pragma unroll
@@ -628,12 +638,12 @@ __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(con
   rhs_source(cs, A, q.b, q.ip, T(damping_rate(cs, A.t, q.x)), ht, Ct, D, msrc);
   if (A.matter) {
 #pragma unroll
-    for (int v = 0; v < NC; ++v) msrc[v] += T(cfo[(CF_M0 + v) * A.npts]);
+    for (int v = 0; v < NC; ++v) msrc[v] += T(cfo[(CF_M0 + v) * A.ncoef]);
   }
   if (!layer) {
 #pragma unroll
-    for (int v = 0; v < NC; ++v) cfo[(CF_M0 + v) * A.npts] = msrc[v];
-    cfo[CF_W * A.npts] = 1.0;
+    for (int v = 0; v < NC; ++v) cfo[(CF_M0 + v) * A.ncoef] = msrc[v];
+    cfo[CF_W * A.ncoef] = 1.0;
     return;
   }
   // the layer's Pi half: w msrc + T, T = (1 - w) d_t Pi_target - rho (Pi - Pi_target) parked at
@@ -642,9 +652,9 @@ __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(con
     const double* dT = MODE == MODE_DU ? ed.d + NC * S : es.nx + NC * sv;
     const long sT = MODE == MODE_DU ? S : sv;
 #pragma unroll
-    for (int v = 0; v < NC; ++v) cfo[(CF_M0 + v) * A.npts] = fma(w, (double)msrc[v], dT[v * sT]);
+    for (int v = 0; v < NC; ++v) cfo[(CF_M0 + v) * A.ncoef] = fma(w, (double)msrc[v], dT[v * sT]);
   }
-  cfo[CF_W * A.npts] = w;
+  cfo[CF_W * A.ncoef] = w;
 }
 
 // Step 4 (src/evolution.jl:324-354): per component v the stencils of h_v and Pi_v
@@ -656,31 +666,32 @@ __global__ void __launch_bounds__(128, MB) rhs_pi_kernel(const Case cs, const Rh
   const RhsArgs A = fixed_geometry<Q, N1S>(A0);
   const long p = A.p0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= A.p1) return;
-  const double* cfi = A.coef + p;
-  const double w = cfi[CF_W * A.npts];
-  if (w < 0.0) return;
   const PointIdx q = point_index(A, p);
+  const double* cfi = A.coef + q.cp;
+  const double w = cfi[CF_W * A.ncoef];
+  if (w < 0.0) return;
+  const long SX = (long)A.NX * A.N1 * A.N1;
   const long S = (long)A.N1 * A.N1 * A.N1;
   const long sv = (long)A.Wx * A.Wd * A.Wd;
   const long s1 = 1, s2 = A.Wx, s3 = (long)A.Wx * A.Wd;
   const double* wk = A.work + q.wo;
   const double inv_h = 1.0 / q.h;
   const T ih = T(inv_h), ih2 = T(inv_h * inv_h);
-  const T b0 = T(cfi[CF_B0 * A.npts]), b1 = T(cfi[CF_B1 * A.npts]), b2 = T(cfi[CF_B2 * A.npts]);
-  const T divb = T(cfi[CF_DIVB * A.npts]);
-  const T da0 = T(cfi[CF_DA0 * A.npts]), da1 = T(cfi[CF_DA1 * A.npts]), da2 = T(cfi[CF_DA2 * A.npts]);
-  const T Axx = T(cfi[CF_AXX * A.npts]), Axy = T(cfi[CF_AXY * A.npts]), Axz = T(cfi[CF_AXZ * A.npts]);
-  const T Ayy = T(cfi[CF_AYY * A.npts]), Ayz = T(cfi[CF_AYZ * A.npts]), Azz = T(cfi[CF_AZZ * A.npts]);
-  const T eh = T(cfi[CF_EH * A.npts]);
+  const T b0 = T(cfi[CF_B0 * A.ncoef]), b1 = T(cfi[CF_B1 * A.ncoef]), b2 = T(cfi[CF_B2 * A.ncoef]);
+  const T divb = T(cfi[CF_DIVB * A.ncoef]);
+  const T da0 = T(cfi[CF_DA0 * A.ncoef]), da1 = T(cfi[CF_DA1 * A.ncoef]), da2 = T(cfi[CF_DA2 * A.ncoef]);
+  const T Axx = T(cfi[CF_AXX * A.ncoef]), Axy = T(cfi[CF_AXY * A.ncoef]), Axz = T(cfi[CF_AXZ * A.ncoef]);
+  const T Ayy = T(cfi[CF_AYY * A.ncoef]), Ayz = T(cfi[CF_AYZ * A.ncoef]), Azz = T(cfi[CF_AZZ * A.ncoef]);
+  const T eh = T(cfi[CF_EH * A.ncoef]);
   EmitDu ed{A.du + (long)q.b * NV * S + q.ip, S};
-  EmitStage es{A.acc + (long)q.b * NV * S + q.ip, A.next + q.wo, A.u0 + q.wo, S, sv, A.ca, A.cb, A.stage};
+  EmitStage es{A.acc + q.ap, A.next + q.wo, A.u0 + q.wo, SX, sv, A.ca, A.cb, A.stage};
 #pragma unroll 1
   for (int v = 0; v < NC; ++v) {
     // the epilogue's loads first: they are in flight while the stencils are formed
-    const double m = cfi[(CF_M0 + v) * A.npts];
+    const double m = cfi[(CF_M0 + v) * A.ncoef];
     double kh = 0.0, uh = 0.0, up = 0.0, ah = 0.0, ap = 0.0;
     if (MODE == MODE_STAGE) {
-      kh = cfi[(CF_DTH0 + v) * A.npts];
+      kh = cfi[(CF_DTH0 + v) * A.ncoef];
       uh = es.pre_u(v);
       up = es.pre_u(NC + v);
       ah = es.pre_a(v);

@@ -2,22 +2,23 @@
 // into shared memory by the Tensor Memory Accelerator: the B200 form of rhs_pi_kernel for
 // blocks of N = 32 cells at q = 4.
 //
-// A CTA owns a tile of one block: the whole x extent (33 points), 11 rows in y and 2 planes
-// in z (3 x 17 = 51 tiles per block; the last z tile's second plane lies past the block and is
-// computed and dropped). 12 warps per CTA: 3 per SM sub-partition leave 168 registers a thread,
-// enough for two points' coefficients without spilling. For each component v in turn, one thread
-// issues two tiled tensor copies of the block's working array into shared memory:
-//   h_v   x -2..47, the tile's rows and planes widened by SR = 2 (50 x 15 x 6 doubles)
-//   Pi_v  x -2..47, widened by KR = 3 for the dissipation      (50 x 17 x 8 doubles)
-// completing on an mbarrier; two such stages alternate, so that the copies of component v + 1
-// run while component v is computed. The boxes are 50 doubles wide (the rows used are 44): a
-// row pitch of 25 sixteen-byte units, 1 modulo the 8 bank groups of a 128-byte shared-memory
-// wavefront, keeps the 16-byte loads of a warp whose lanes cross from one row to the next free
-// of bank conflicts. Each thread computes two neighbouring points along x,
-// (i0, i0 + 1) with i0 = -1, 1, ..., 31, from 16-byte shared-memory loads: one load serves
-// both points of every y and z tap and two x taps, so a point costs about 34 shared loads per
-// component against the 80 global loads of the one-point kernel. The point i = -1 of the first
-// pair is a ghost: it is computed and dropped.
+// A persistent CTA of 12 warps works through tiles of the blocks: NP pairs of neighbouring points
+// along x (the whole row) x TY rows x TZ planes. For each component v of a tile one thread issues two
+// tiled tensor copies of the block's working array into shared memory, whole rows (x -4 .. 35):
+//   h_v   the tile's rows and planes widened by SR = 2
+//   Pi_v  widened by KR = 3 for the dissipation
+// completing on an mbarrier; two such stages alternate, so that the copies of the next component (of
+// the next tile after the last one) run while component v is computed. Each thread computes the two
+// points (i0, i0 + 1), i0 = 0, 2, ..., from 16-byte shared loads: one load serves both points of
+// every y and z tap and two x taps. A row's owned points start on a sector (row_lead), so the pairs'
+// global loads and stores are 16 bytes too.
+//
+// The mixed derivatives are outer sums of inner sums: d_x d_y h = sum_a w_a D_y h(x + a), d_x d_z h and
+// d_y d_z h outer sums of D_z h. An inner sum is formed once, by the thread that owns the pair (those
+// beyond the tile by extra tasks), and read by the points around it from shared memory: 39 instead of 91
+// FP64 operations a point and component, and 45 instead of 68 shared loads a pair, against forming them
+// at each point. On 64 blocks a stage takes 691 us (777 us with every inner sum formed where it is used);
+// it is bound by DRAM (3.0 GB, 4.3 TB/s) and by shared-load latency at 12 warps an SM.
 //
 // The arithmetic is the one-point kernel's, operation for operation (the same stencil sums in
 // the same order and the same contraction with the head's coefficients), so both kernels give
@@ -25,413 +26,382 @@
 //
 // Waits on the mbarriers are bounded: a wait that gives up records TGH_ERR_TIMEOUT in the
 // launch's status word, waits (bounded again) for the copies it issued to land, and the CTA
-// returns without writing; the host reads the word after the step.
+// returns without writing further; the host reads the word after the step.
 #pragma once
-#include <cuda.h>
-
 #include "rhs.cuh"
+#include "tma.cuh"
 
 namespace tgh {
 
 namespace pitma {
 constexpr int N1 = 33, G = 3, SR = 2, KR = 3;  // q = 4, N = 32
-constexpr int TY = 11, TZ = 2, NPAIR = 17;
-constexpr int XB = 50;                                   // box width: x = -2 .. 47 (see below)
-constexpr int HY = TY + 2 * SR, HZ = TZ + 2 * SR;          // 15, 6
-constexpr int PY = TY + 2 * KR, PZ = TZ + 2 * KR;        // 17, 8
-constexpr int HN = XB * HY * HZ, PN = XB * PY * PZ;      // doubles per box
-constexpr int HBYTES = HN * 8, PBYTES = PN * 8;
-constexpr int HOFF = 0;                                  // byte offsets inside one stage
-constexpr int POFF = ((HBYTES + 127) / 128) * 128;
-constexpr int STAGE = ((POFF + PBYTES + 127) / 128) * 128;
-constexpr int SMEM = 2 * STAGE + 256;                    // two stages, the mbarriers, alignment
-constexpr int THREADS = 384;                             // 17 x 11 x 2 = 374 pair threads, 12 warps
-constexpr int TILESY = N1 / TY, TILESZ = (N1 + TZ - 1) / TZ;
-constexpr int TILES = TILESY * TILESZ;                   // 3 x 17 = 51 per block
-static_assert(N1 % TY == 0, "the y tiles cover a block exactly");
+constexpr int XB = 40, XC = 4;                 // the boxes' rows, and the column of point i = 0
+constexpr int THREADS = 384;
+// one tile shape: pairs along x, rows, planes; its boxes and inner-sum arrays in doubles
+template <int NP_, int TY_, int TZ_> struct Shape {
+  static constexpr int NP = NP_, TY = TY_, TZ = TZ_, ROWS = TY * TZ;
+  static constexpr int HY = TY + 2 * SR, HZ = TZ + 2 * SR, PY = TY + 2 * KR, PZ = TZ + 2 * KR;
+  static constexpr int HN = XB * HY * HZ, PN = XB * PY * PZ;
+  static constexpr int DY = TY + 2 * SR;                        // rows of D_z per plane
+  static constexpr int DN = XB * ROWS + XB * DY * TZ;           // D_y, then D_z
+  static constexpr int NE = 4 * ROWS + 2 * SR * TZ * NP;        // inner-sum pairs beyond the tile's own
+  static_assert(NP * ROWS <= THREADS && NE <= THREADS, "a thread per pair and per extra inner sum");
+};
+// whole blocks: 33 points a row, 33 = 3 x 11 rows, 17 x 2 planes (the last one past the block)
+using Whole = Shape<17, 11, 2>;
+constexpr int STAGE = (Whole::HN + Whole::PN) * 8;
+constexpr int DBYTES = Whole::DN * 8;
+constexpr int SMEM = 2 * STAGE + DBYTES + 16 + 128;             // two stages, inner sums, mbarriers, alignment
+static_assert(STAGE % 128 == 0 && (Whole::HN * 8) % 128 == 0, "the copies land on 128-byte boundaries");
 static_assert(SMEM <= 227 * 1024, "two stages fit in shared memory");
+constexpr int TILESY = N1 / Whole::TY, TILESZ = (N1 + Whole::TZ - 1) / Whole::TZ;
+constexpr int TILES = TILESY * TILESZ;                          // 3 x 17 = 51 per block
 }  // namespace pitma
 
-// The tensor maps one launch reads: the working array viewed as 4-d (x, y, z, block x 20 +
-// variable), with the h box and the Pi box.
-struct PiTmaMaps {
-  CUtensorMap h, pi;
-};
-
-struct PiTmaStatus {
-  int* err;         // TGH_ERR_TIMEOUT is stored here by a wait that gives up
-  long long limit;  // polls a wait may make (negative: give up at once, which tests use)
-};
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait on one phase of an mbarrier: false when it gave up
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, long long limit) {
-  for (long long it = 0; it <= limit; ++it)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-__device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map, int x, int y, int z, int c,
-                                            unsigned bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];" ::"r"(dst),
-      "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(c), "r"(bar)
-      : "memory");
-}
-
-// issue component v's two boxes for tile (b, y0, z0) into stage st
-__device__ __forceinline__ void pitma_issue(const PiTmaMaps& M, unsigned base, unsigned bar, int st, int b, int v,
-                                           int y0, int z0) {
+// issue component v's two boxes for tile (b, y0, z0) into the stage at s
+template <class Sh>
+__device__ __forceinline__ void pitma_issue(const TmaMaps& M, unsigned s, unsigned bar, int b, int v, int y0, int z0) {
   using namespace pitma;
-  const unsigned s = base + st * STAGE;
-  mbar_expect_tx(bar, HBYTES + PBYTES);
+  mbar_expect_tx(bar, (Sh::HN + Sh::PN) * 8);
   // h: rows y0 + G - SR .., planes z0 + G - SR ..; Pi: widened by KR
-  tma_load_4d(s + HOFF, &M.h, -2, y0 + G - SR, z0 + G - SR, b * NV + v, bar);
-  tma_load_4d(s + POFF, &M.pi, -2, y0 + G - KR, z0 + G - KR, b * NV + NC + v, bar);
+  tma_load_4d(s, &M.h, 0, y0 + G - SR, z0 + G - SR, b * NV + v, bar);
+  tma_load_4d(s + Sh::HN * 8, &M.pi, 0, y0 + G - KR, z0 + G - KR, b * NV + NC + v, bar);
+}
+
+__device__ __forceinline__ double2 lds2(const double* p) { return *reinterpret_cast<const double2*>(p); }
+__device__ __forceinline__ double2 ldg2(const double* p) { return *reinterpret_cast<const double2*>(p); }
+
+// the inner sums of the mixed differences at the pair p along stride s (the reference's sum term by
+// term, st_mixed_ref); r returns the four pairs read
+__device__ __forceinline__ double2 inner_sum(const double* p, int s, double2 r[2 * pitma::SR]) {
+  using namespace pitma;
+  double2 in;
+#pragma unroll
+  for (int n = 0; n < 2 * SR; ++n) {
+    const int e = n < SR ? n - SR : n - SR + 1;
+    r[n] = lds2(p + e * s);
+    const double t0 = __dmul_rn(d1s<4>(e), r[n].x), t1 = __dmul_rn(d1s<4>(e), r[n].y);
+    in.x = n == 0 ? t0 : __dadd_rn(in.x, t0);
+    in.y = n == 0 ? t1 : __dadd_rn(in.y, t1);
+  }
+  return in;
+}
+// first (paired, fused) and second (term by term) differences of the pair from its four neighbours and centre
+__device__ __forceinline__ void pair_d1_d2(const double2 r[2 * pitma::SR], double2 c, double d1[2], double d2[2]) {
+  using namespace pitma;
+  d1[0] = d1[1] = 0.0;
+#pragma unroll
+  for (int k = 1; k <= SR; ++k) {
+    d1[0] = fma(W<4>::d1(k), r[SR - 1 + k].x - r[SR - k].x, d1[0]);
+    d1[1] = fma(W<4>::d1(k), r[SR - 1 + k].y - r[SR - k].y, d1[1]);
+  }
+  d2[0] = __dmul_rn(W<4>::d2(SR), r[0].x);
+  d2[1] = __dmul_rn(W<4>::d2(SR), r[0].y);
+#pragma unroll
+  for (int k = -SR + 1; k <= SR; ++k) {
+    const double2 u = k == 0 ? c : r[k < 0 ? k + SR : k + SR - 1];
+    const double w = W<4>::d2(k < 0 ? -k : k);
+    d2[0] = __dadd_rn(d2[0], __dmul_rn(w, u.x));
+    d2[1] = __dadd_rn(d2[1], __dmul_rn(w, u.y));
+  }
+}
+// outer sum over a row's x offsets of the inner sums around the pair at p (both points)
+__device__ __forceinline__ void outer_x(const double* p, double out[2]) {
+  using namespace pitma;
+  double r[6];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const double2 q = lds2(p - 2 + 2 * t);
+    r[2 * t] = q.x;
+    r[2 * t + 1] = q.y;
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    double o = __dmul_rn(d1s<4>(-SR), r[e]);
+#pragma unroll
+    for (int a = -SR + 1; a <= SR; ++a) {
+      if (a == 0) continue;
+      o = __dadd_rn(o, __dmul_rn(d1s<4>(a), r[2 + e + a]));
+    }
+    out[e] = o;
+  }
 }
 
 template <bool DISS, int MODE>
 __global__ void __launch_bounds__(pitma::THREADS)
-    rhs_pi_tma_kernel(const Case cs, const RhsArgs A, const __grid_constant__ PiTmaMaps M, const PiTmaStatus stat,
-                      int b0) {
+    rhs_pi_tma_kernel(const RhsArgs A, const __grid_constant__ TmaMaps M, const WaitStatus stat, int b0,
+                      int ntiles) {
   using namespace pitma;
+  using Sh = Whole;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int b = b0 + blockIdx.x / TILES;
-  const int tile = blockIdx.x % TILES;
-  const int y0 = (tile % TILESY) * TY, z0 = (tile / TILESY) * TZ;
   // the copies land on 128-byte boundaries
   const unsigned raw = smem_u32(smem_raw);
   const unsigned base = (raw + 127u) & ~127u;
   unsigned char* smem = smem_raw + (base - raw);
-  const unsigned bar0 = base + 2 * STAGE, bar1 = bar0 + 8;
+  double* Dy = reinterpret_cast<double*>(smem + 2 * STAGE);
+  double* Dz = Dy + XB * Sh::ROWS;
+  const unsigned bar0 = base + 2 * STAGE + DBYTES;
   const int tid = threadIdx.x;
+  // the CTA's tiles blockIdx.x, blockIdx.x + gridDim.x, ...; component v of its m-th tile is copy
+  // n = 10 m + v, into stage n & 1, the mbarrier's phase n >> 1
+  auto issue = [&](int n) {
+    const int tile = blockIdx.x + (n / NC) * gridDim.x;
+    if (tile >= ntiles) return;
+    const int t = tile % TILES;
+    pitma_issue<Sh>(M, base + (n & 1) * STAGE, bar0 + 8 * (n & 1), b0 + tile / TILES, n % NC, (t % TILESY) * Sh::TY,
+                    (t / TILESY) * Sh::TZ);
+  };
   if (tid == 0) {
     mbar_init(bar0, 1);
-    mbar_init(bar1, 1);
+    mbar_init(bar0 + 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    pitma_issue(M, base, bar0, 0, b, 0, y0, z0);
-    pitma_issue(M, base, bar1, 1, b, 1, y0, z0);
+    issue(0);
+    issue(1);
   }
   __syncthreads();
 
-  // this thread's pair: x = i0, i0 + 1 (i0 = -1, 1, ..., 31), row j, plane k of the block
-  const bool active = tid < NPAIR * TY * TZ;
-  const int ip = tid % NPAIR, jj = (tid / NPAIR) % TY, kk = tid / (NPAIR * TY);
-  const int i0 = 2 * ip - 1;
-  const int j = y0 + jj, k = z0 + kk;
-  const int sx = i0 + G + 2;                      // shared column of point i0 (even)
-  const int cH = sx + XB * ((jj + SR) + HY * (kk + SR));
-  const int cP = sx + XB * ((jj + KR) + PY * (kk + KR));
-  const long S = (long)N1 * N1;
-  const long S3 = S * N1;
-  const int Wd = N1 + 2 * G, Wx = Wd + 1;
-  const long sv = (long)Wx * Wd * Wd;
-  // the two points: state index, working index, and whether each is computed here
-  long pidx[2], wo[2];
-  bool own[2];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const int i = i0 + e;
-    own[e] = active && i >= 0 && k < N1;  // the last z tile's second plane lies past the block
-    const int ic = i < 0 ? 0 : i, kc = k < N1 ? k : N1 - 1;
-    pidx[e] = (long)b * S3 + ic + N1 * (j + (long)N1 * kc);
-    wo[e] = (long)b * NV * sv + (ic + G) + (long)Wx * ((j + G) + (long)Wd * (kc + G));
+  // this thread's pair in a tile: points i0, i0 + 1 of row jj, plane kk
+  const bool active = tid < Sh::NP * Sh::ROWS;
+  const int i0 = 2 * (tid % Sh::NP), row = active ? tid / Sh::NP : 0;
+  const int jj = row % Sh::TY, kk = row / Sh::TY;
+  const int cH = i0 + XC + XB * ((jj + SR) + Sh::HY * (kk + SR));
+  const int cP = i0 + XC + XB * ((jj + KR) + Sh::PY * (kk + KR));
+  const int cDy = i0 + XC + XB * row;
+  const int cDz = i0 + XC + XB * ((jj + SR) + Sh::DY * kk);
+  constexpr int s3h = XB * Sh::HY, s3p = XB * Sh::PY;
+  // the extra inner sum this thread forms: D_y, then D_z, one pair beyond each end of the tile's rows, and
+  // D_z on the SR rows either side of the tile
+  int eH = -1, eS = 0;
+  double* eD = nullptr;
+  if (tid < 4 * Sh::ROWS) {
+    const int r = tid / 2 % Sh::ROWS, c = (tid & 1) ? XC + 2 * Sh::NP : XC - 2, j = r % Sh::TY, k = r / Sh::TY;
+    const bool isy = tid < 2 * Sh::ROWS;
+    eH = c + XB * ((j + SR) + Sh::HY * (k + SR));
+    eS = isy ? XB : s3h;
+    eD = isy ? Dy + c + XB * r : Dz + c + XB * ((j + SR) + Sh::DY * k);
+  } else if (tid < Sh::NE) {
+    const int n = tid - 4 * Sh::ROWS, c = XC + 2 * (n % Sh::NP), m = n / Sh::NP;
+    const int jr = m % (2 * SR), k = m / (2 * SR), j = jr < SR ? jr : jr + Sh::TY;  // row j - SR of the tile
+    eH = c + XB * (j + Sh::HY * (k + SR));
+    eS = s3h;
+    eD = Dz + c + XB * (j + Sh::DY * k);
   }
-  const double* cf0 = A.coef + pidx[0];
-  const double* cf1 = A.coef + pidx[1];
-  double w[2];
-  w[0] = own[0] ? cf0[CF_W * A.npts] : -1.0;
-  w[1] = own[1] ? cf1[CF_W * A.npts] : -1.0;
-  const bool live0 = w[0] >= 0.0, live1 = w[1] >= 0.0;
-  double cb[2][14];
-#pragma unroll
-  for (int c = 0; c < 14; ++c) {
-    cb[0][c] = live0 ? cf0[c * A.npts] : 0.0;
-    cb[1][c] = live1 ? cf1[c * A.npts] : 0.0;
-  }
-  const double inv_h = 1.0 / A.blk[8 * b + 3];
-  const double ih = inv_h, ih2 = inv_h * inv_h;
-  const long s2x = XB, s3h = (long)XB * HY, s3p = (long)XB * PY;
-  const double* smd = reinterpret_cast<const double*>(smem);
+
+  constexpr int NX = point_pitch(N1), Wd = N1 + 2 * G, Wx = row_pitch(Wd, G);
+  constexpr long S = (long)N1 * N1 * N1, SX = (long)NX * N1 * N1, sv = (long)Wx * Wd * Wd;
+  static_assert(Wx == XB && row_lead(G) + G == XC, "the boxes are whole rows");
   bool ok = true;
-  int failed_at = 0;
+  int n = 0;  // the copy the CTA waits for next
 
 #pragma unroll 1
-  for (int v = 0; v < NC; ++v) {
-    const int st = v & 1;
-    // the epilogue's loads first: they are in flight while the copies land
-    double m[2], kh[2] = {0, 0}, uh[2] = {0, 0}, up[2] = {0, 0}, ah[2] = {0, 0}, ap[2] = {0, 0};
-    const double* cfs[2] = {cf0, cf1};
-    const bool live[2] = {live0, live1};
+  for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
+    const int b = b0 + tile / TILES, t = tile % TILES;
+    const int j = (t % TILESY) * Sh::TY + jj, k = (t / TILESY) * Sh::TZ + kk;
+    // the last z tile's second plane lies past the block: computed and dropped, as is i = 33
+    const bool own0 = active && k < N1, own1 = own0 && i0 + 1 < N1;
+    const int kc = k < N1 ? k : N1 - 1;
+    const long ic = i0 + (long)NX * (j + (long)N1 * kc);
+    const double* cf = A.coef + (long)b * SX + ic;
+    const double2 ww = own0 ? ldg2(cf + CF_W * A.ncoef) : make_double2(-1.0, -1.0);
+    const double w[2] = {ww.x, own1 ? ww.y : -1.0};
+    const bool live[2] = {w[0] >= 0.0, w[1] >= 0.0};
+    const bool any = live[0] || live[1], both = live[0] && live[1];
+    double cb[2][14];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      m[e] = live[e] ? cfs[e][(CF_M0 + v) * A.npts] : 0.0;
-      if (MODE == MODE_STAGE && live[e]) {
-        kh[e] = cfs[e][(CF_DTH0 + v) * A.npts];
-        if (A.stage != 4) {
-          uh[e] = A.u0[wo[e] + v * sv];
-          up[e] = A.u0[wo[e] + (NC + v) * sv];
-        }
-        if (A.stage != 1) {
-          const long ai = (long)b * NV * S3 + (pidx[e] - (long)b * S3);
-          ah[e] = A.acc[ai + v * S3];
-          ap[e] = A.acc[ai + (NC + v) * S3];
-        }
-      }
+    for (int c = 0; c < 14; ++c) {
+      const double2 q = any ? ldg2(cf + c * A.ncoef) : make_double2(0.0, 0.0);
+      cb[0][c] = live[0] ? q.x : 0.0;
+      cb[1][c] = live[1] ? q.y : 0.0;
     }
-    // every thread waits (bounded) for the stage; the CTA goes on only if all of them saw it.
-    // The vote is also the barrier after component v - 1: its stage may now be refilled with
-    // component v + 1, which lands while v is computed.
-    const bool got = mbar_wait(st ? bar1 : bar0, (v >> 1) & 1, stat.limit);
-    if (!__syncthreads_and(got)) {
-      ok = false;
-      failed_at = v;
-      break;
-    }
-    if (tid == 0 && v >= 1 && v + 1 < NC) pitma_issue(M, base, st ? bar0 : bar1, st ^ 1, b, v + 1, y0, z0);
-    const double* H = smd + (st * STAGE + HOFF) / 8;
-    const double* P = smd + (st * STAGE + POFF) / 8;
-    double s[2], p2[2];
-    if (active) {
-      // ---- Pi_v: x taps from five 16-byte loads (columns sx - 4 .. sx + 5) ----
-      const double* pc = P + cP;
-      double px[10];
-#pragma unroll
-      for (int t = 0; t < 5; ++t) {
-        const double2 q = *reinterpret_cast<const double2*>(pc - 4 + 2 * t);
-        px[2 * t] = q.x;
-        px[2 * t + 1] = q.y;
+    const double ih = 1.0 / A.blk[8 * b + 3], ih2 = ih * ih;
+    const long wo = (long)b * NV * sv + (i0 + G) + (long)Wx * ((j + G) + (long)Wd * (kc + G));
+    double* acc = MODE == MODE_STAGE ? A.acc + (long)b * NV * SX + ic : nullptr;
+    double* du = MODE == MODE_DU ? A.du + (long)b * NV * S + i0 + N1 * (j + (long)N1 * kc) : nullptr;
+
+#pragma unroll 1
+    for (int v = 0; v < NC; ++v, ++n) {
+      // the epilogue's loads first: they are in flight while the copies land
+      double2 m = make_double2(0, 0), kh = m, uh = m, up = m, ah = m, ap = m;
+      if (any) {
+        m = ldg2(cf + (CF_M0 + v) * A.ncoef);
+        if (MODE == MODE_STAGE) {
+          kh = ldg2(cf + (CF_DTH0 + v) * A.ncoef);
+          if (A.stage != 4) {
+            uh = ldg2(A.u0 + wo + v * sv);
+            up = ldg2(A.u0 + wo + (NC + v) * sv);
+          }
+          if (A.stage != 1) {
+            ah = ldg2(acc + v * SX);
+            ap = ldg2(acc + (NC + v) * SX);
+          }
+        }
       }
-      // point e sits at px[4 + e]
-      double pcen[2], d1x[2], kox[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double* u = px + 4 + e;
-        pcen[e] = u[0];
-        double a = 0.0;
-#pragma unroll
-        for (int kx = 1; kx <= SR; ++kx) a = fma(W<4>::d1(kx), u[kx] - u[-kx], a);
-        d1x[e] = a;
-        double c = W<4>::ko(0) * u[0];
-#pragma unroll
-        for (int kx = 1; kx <= KR; ++kx) c = fma(W<4>::ko(kx), u[kx] + u[-kx], c);
-        kox[e] = c;
+      // every thread waits (bounded) for the stage; the CTA goes on only if all of them saw it.
+      // The vote is also the barrier after the component before: its stage and the inner sums may
+      // now be refilled.
+      const bool got = mbar_wait(bar0 + 8 * (n & 1), (n >> 1) & 1, stat.limit);
+      if (!__syncthreads_and(got)) {
+        ok = false;
+        break;
       }
-      // y and z taps: one 16-byte load per offset serves both points
-      double d1y[2] = {0, 0}, d1z[2] = {0, 0}, koy[2], koz[2];
-      koy[0] = W<4>::ko(0) * pcen[0];
-      koy[1] = W<4>::ko(0) * pcen[1];
-      koz[0] = koy[0];
-      koz[1] = koy[1];
-      double2 yp[KR + 1], ym[KR + 1], zp[KR + 1], zm[KR + 1];
-#pragma unroll
-      for (int kt = 1; kt <= KR; ++kt) {
-        yp[kt] = *reinterpret_cast<const double2*>(pc + kt * s2x);
-        ym[kt] = *reinterpret_cast<const double2*>(pc - kt * s2x);
-        zp[kt] = *reinterpret_cast<const double2*>(pc + kt * s3p);
-        zm[kt] = *reinterpret_cast<const double2*>(pc - kt * s3p);
-      }
-#pragma unroll
-      for (int kt = 1; kt <= SR; ++kt) {
-        d1y[0] = fma(W<4>::d1(kt), yp[kt].x - ym[kt].x, d1y[0]);
-        d1y[1] = fma(W<4>::d1(kt), yp[kt].y - ym[kt].y, d1y[1]);
-        d1z[0] = fma(W<4>::d1(kt), zp[kt].x - zm[kt].x, d1z[0]);
-        d1z[1] = fma(W<4>::d1(kt), zp[kt].y - zm[kt].y, d1z[1]);
-      }
-#pragma unroll
-      for (int kt = 1; kt <= KR; ++kt) {
-        koy[0] = fma(W<4>::ko(kt), yp[kt].x + ym[kt].x, koy[0]);
-        koy[1] = fma(W<4>::ko(kt), yp[kt].y + ym[kt].y, koy[1]);
-        koz[0] = fma(W<4>::ko(kt), zp[kt].x + zm[kt].x, koz[0]);
-        koz[1] = fma(W<4>::ko(kt), zp[kt].y + zm[kt].y, koz[1]);
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double* c = cb[e];
-        double a = c[CF_B0] * (ih * d1x[e]);
-        a = fma(c[CF_B1], ih * d1y[e], a);
-        a = fma(c[CF_B2], ih * d1z[e], a);
-        s[e] = fma(c[CF_DIVB], pcen[e], a);
-      }
-      // ---- h_v: x taps from three loads (columns sx - 2 .. sx + 3) ----
+      if (tid == 0 && n >= 1) issue(n + 1);
+      const double* H = reinterpret_cast<const double*>(smem + (n & 1) * STAGE);
+      const double* P = H + Sh::HN;
+      double s[2], p2[2], hd1[3][2], ko[2];
+      // ---- h_v: the y and z taps give the inner sums and the y, z differences ----
       const double* hc = H + cH;
-      double hx[6];
-#pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        const double2 q = *reinterpret_cast<const double2*>(hc - 2 + 2 * t);
-        hx[2 * t] = q.x;
-        hx[2 * t + 1] = q.y;
-      }
-      // first differences paired at +-k with fused multiply-adds, second differences as the
-      // reference's sums term by term (st_d2_ref, st_mixed_ref: lowest offset first, every
-      // product and sum rounded on its own), so that they carry the reference's bits
-      double hcen[2], hd1x[2], hd2x[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double* u = hx + 2 + e;
-        hcen[e] = u[0];
-        double a = 0.0;
-#pragma unroll
-        for (int kx = 1; kx <= SR; ++kx) a = fma(W<4>::d1(kx), u[kx] - u[-kx], a);
-        hd1x[e] = a;
-        double c = __dmul_rn(W<4>::d2(SR), u[-SR]);
-#pragma unroll
-        for (int kx = -SR + 1; kx <= SR; ++kx) c = __dadd_rn(c, __dmul_rn(W<4>::d2(kx < 0 ? -kx : kx), u[kx]));
-        hd2x[e] = c;
-      }
-      double hd1y[2] = {0, 0}, hd1z[2] = {0, 0}, hd2y[2], hd2z[2];
       {
-        double2 ry[2 * SR + 1], rz[2 * SR + 1];  // rows y + k and planes z + k, k = -SR .. SR
+        double hx[6];
 #pragma unroll
-        for (int k = -SR; k <= SR; ++k) {
-          if (k == 0) continue;
-          ry[k + SR] = *reinterpret_cast<const double2*>(hc + k * s2x);
-          rz[k + SR] = *reinterpret_cast<const double2*>(hc + k * s3h);
+        for (int q = 0; q < 3; ++q) {
+          const double2 r = lds2(hc - 2 + 2 * q);
+          hx[2 * q] = r.x;
+          hx[2 * q + 1] = r.y;
         }
-        ry[SR] = rz[SR] = make_double2(hcen[0], hcen[1]);
+        const double2 c = make_double2(hx[2], hx[3]);
+        double2 r[2 * SR];
+        double d2[2];
+        const double2 iy = inner_sum(hc, XB, r);
+        if (active) *reinterpret_cast<double2*>(Dy + cDy) = iy;
+        pair_d1_d2(r, c, hd1[1], d2);
+        p2[0] = d2[0];
+        p2[1] = d2[1];
+        const double2 iz = inner_sum(hc, s3h, r);
+        if (active) *reinterpret_cast<double2*>(Dz + cDz) = iz;
+        pair_d1_d2(r, c, hd1[2], d2);
+        // x: first differences paired at +-k, second differences term by term
 #pragma unroll
-        for (int kt = 1; kt <= SR; ++kt) {
-          hd1y[0] = fma(W<4>::d1(kt), ry[SR + kt].x - ry[SR - kt].x, hd1y[0]);
-          hd1y[1] = fma(W<4>::d1(kt), ry[SR + kt].y - ry[SR - kt].y, hd1y[1]);
-          hd1z[0] = fma(W<4>::d1(kt), rz[SR + kt].x - rz[SR - kt].x, hd1z[0]);
-          hd1z[1] = fma(W<4>::d1(kt), rz[SR + kt].y - rz[SR - kt].y, hd1z[1]);
-        }
-        const double wR = W<4>::d2(SR);
-        hd2y[0] = __dmul_rn(wR, ry[0].x);
-        hd2y[1] = __dmul_rn(wR, ry[0].y);
-        hd2z[0] = __dmul_rn(wR, rz[0].x);
-        hd2z[1] = __dmul_rn(wR, rz[0].y);
+        for (int e = 0; e < 2; ++e) {
+          const double* u = hx + 2 + e;
+          double a = 0.0;
 #pragma unroll
-        for (int k = -SR + 1; k <= SR; ++k) {
-          const double wk = W<4>::d2(k < 0 ? -k : k);
-          hd2y[0] = __dadd_rn(hd2y[0], __dmul_rn(wk, ry[k + SR].x));
-          hd2y[1] = __dadd_rn(hd2y[1], __dmul_rn(wk, ry[k + SR].y));
-          hd2z[0] = __dadd_rn(hd2z[0], __dmul_rn(wk, rz[k + SR].x));
-          hd2z[1] = __dadd_rn(hd2z[1], __dmul_rn(wk, rz[k + SR].y));
+          for (int kx = 1; kx <= SR; ++kx) a = fma(W<4>::d1(kx), u[kx] - u[-kx], a);
+          hd1[0][e] = a;
+          double d = __dmul_rn(W<4>::d2(SR), u[-SR]);
+#pragma unroll
+          for (int kx = -SR + 1; kx <= SR; ++kx) d = __dadd_rn(d, __dmul_rn(W<4>::d2(kx < 0 ? -kx : kx), u[kx]));
+          double q = cb[e][CF_AXX] * d;
+          q = fma(cb[e][CF_AYY], p2[e], q);
+          p2[e] = fma(cb[e][CF_AZZ], d2[e], q);
         }
       }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double* c = cb[e];
-        s[e] = fma(c[CF_DA0], ih * hd1x[e], s[e]);
-        s[e] = fma(c[CF_DA1], ih * hd1y[e], s[e]);
-        s[e] = fma(c[CF_DA2], ih * hd1z[e], s[e]);
-        double a = c[CF_AXX] * hd2x[e];
-        a = fma(c[CF_AYY], hd2y[e], a);
-        p2[e] = fma(c[CF_AZZ], hd2z[e], a);
+      if (eH >= 0) {
+        double2 r[2 * SR];
+        *reinterpret_cast<double2*>(eD) = inner_sum(H + eH, eS, r);
       }
-      // mixed x-y and x-z: outer sum over the x offsets a, inner over the y rows (z planes)
-      // e; each row (plane) e, from three loads, serves every a of both points
-      double mxy[2], mxz[2], myz[2];
+      // ---- Pi_v: x taps from five 16-byte loads, y and z taps one load an offset ----
+      {
+        const double* pc = P + cP;
+        double px[10];
 #pragma unroll
-      for (int pl = 0; pl < 2; ++pl) {
-        const long se = pl == 0 ? s2x : s3h;
-        double in[2][2 * SR];  // [point][a = -SR .. -1, 1 .. SR]
+        for (int q = 0; q < 5; ++q) {
+          const double2 r = lds2(pc - 4 + 2 * q);
+          px[2 * q] = r.x;
+          px[2 * q + 1] = r.y;
+        }
+        double d1[3][2], kd[3][2];
 #pragma unroll
-        for (int e = -SR; e <= SR; ++e) {
-          if (e == 0) continue;
-          double r[6];  // x - 2 .. x + 3 of row (plane) e
+        for (int e = 0; e < 2; ++e) {
+          const double* u = px + 4 + e;
+          double a = 0.0;
 #pragma unroll
-          for (int t = 0; t < 3; ++t) {
-            const double2 q = *reinterpret_cast<const double2*>(hc - 2 + 2 * t + e * se);
-            r[2 * t] = q.x;
-            r[2 * t + 1] = q.y;
-          }
-          const double we = d1s<4>(e);
+          for (int kx = 1; kx <= SR; ++kx) a = fma(W<4>::d1(kx), u[kx] - u[-kx], a);
+          d1[0][e] = a;
+          double c = W<4>::ko(0) * u[0];
+          kd[1][e] = kd[2][e] = c;
 #pragma unroll
-          for (int pt = 0; pt < 2; ++pt)
+          for (int kx = 1; kx <= KR; ++kx) c = fma(W<4>::ko(kx), u[kx] + u[-kx], c);
+          kd[0][e] = c;
+        }
 #pragma unroll
-            for (int ia = 0; ia < 2 * SR; ++ia) {
-              const int a = ia < SR ? ia - SR : ia - SR + 1;
-              const double term = __dmul_rn(we, r[2 + pt + a]);
-              in[pt][ia] = e == -SR ? term : __dadd_rn(in[pt][ia], term);
+        for (int ax = 1; ax < 3; ++ax) {
+          const int st = ax == 1 ? XB : s3p;
+          d1[ax][0] = d1[ax][1] = 0.0;
+#pragma unroll
+          for (int kt = 1; kt <= KR; ++kt) {
+            const double2 up2 = lds2(pc + kt * st), dn2 = lds2(pc - kt * st);
+            if (kt <= SR) {
+              d1[ax][0] = fma(W<4>::d1(kt), up2.x - dn2.x, d1[ax][0]);
+              d1[ax][1] = fma(W<4>::d1(kt), up2.y - dn2.y, d1[ax][1]);
             }
-        }
-#pragma unroll
-        for (int pt = 0; pt < 2; ++pt) {
-          double o = __dmul_rn(d1s<4>(-SR), in[pt][0]);
-#pragma unroll
-          for (int ia = 1; ia < 2 * SR; ++ia) {
-            const int a = ia < SR ? ia - SR : ia - SR + 1;
-            o = __dadd_rn(o, __dmul_rn(d1s<4>(a), in[pt][ia]));
+            kd[ax][0] = fma(W<4>::ko(kt), up2.x + dn2.x, kd[ax][0]);
+            kd[ax][1] = fma(W<4>::ko(kt), up2.y + dn2.y, kd[ax][1]);
           }
-          if (pl == 0) mxy[pt] = o;
-          else mxz[pt] = o;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double* c = cb[e];
+          double a = c[CF_B0] * (ih * d1[0][e]);
+          a = fma(c[CF_B1], ih * d1[1][e], a);
+          a = fma(c[CF_B2], ih * d1[2][e], a);
+          a = fma(c[CF_DIVB], px[4 + e], a);
+          a = fma(c[CF_DA0], ih * hd1[0][e], a);
+          a = fma(c[CF_DA1], ih * hd1[1][e], a);
+          s[e] = fma(c[CF_DA2], ih * hd1[2][e], a);
+          ko[e] = kd[0][e] + kd[1][e] + kd[2][e];
         }
       }
-      // mixed y-z: outer sum over the y rows a, inner over the z planes e
+      __syncthreads();  // the inner sums are written
+      {
+        double mxy[2], mxz[2], myz[2];
+        outer_x(Dy + cDy, mxy);
+        outer_x(Dz + cDz, mxz);
 #pragma unroll
-      for (int a = -SR; a <= SR; ++a) {
-        if (a == 0) continue;
-        double in0 = 0.0, in1 = 0.0;
-#pragma unroll
-        for (int e = -SR; e <= SR; ++e) {
-          if (e == 0) continue;
-          const double2 q = *reinterpret_cast<const double2*>(hc + a * s2x + e * s3h);
-          const double t0 = __dmul_rn(d1s<4>(e), q.x), t1 = __dmul_rn(d1s<4>(e), q.y);
-          in0 = e == -SR ? t0 : __dadd_rn(in0, t0);
-          in1 = e == -SR ? t1 : __dadd_rn(in1, t1);
+        for (int a = -SR; a <= SR; ++a) {
+          if (a == 0) continue;
+          const double2 q = lds2(Dz + cDz + a * XB);
+          const double o0 = __dmul_rn(d1s<4>(a), q.x), o1 = __dmul_rn(d1s<4>(a), q.y);
+          myz[0] = a == -SR ? o0 : __dadd_rn(myz[0], o0);
+          myz[1] = a == -SR ? o1 : __dadd_rn(myz[1], o1);
         }
-        const double o0 = __dmul_rn(d1s<4>(a), in0), o1 = __dmul_rn(d1s<4>(a), in1);
-        myz[0] = a == -SR ? o0 : __dadd_rn(myz[0], o0);
-        myz[1] = a == -SR ? o1 : __dadd_rn(myz[1], o1);
-      }
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double* c = cb[e];
-        double q = fma(c[CF_AXY], mxy[e], p2[e]);
-        q = fma(c[CF_AXZ], mxz[e], q);
-        q = fma(c[CF_AYZ], myz[e], q);
-        s[e] = fma(ih2, q, s[e]);
-        if (DISS) s[e] = fma(c[CF_EH], kox[e] + koy[e] + koz[e], s[e]);
+        for (int e = 0; e < 2; ++e) {
+          const double* c = cb[e];
+          double q = fma(c[CF_AXY], mxy[e], p2[e]);
+          q = fma(c[CF_AXZ], mxz[e], q);
+          q = fma(c[CF_AYZ], myz[e], q);
+          s[e] = fma(ih2, q, s[e]);
+          if (DISS) s[e] = fma(c[CF_EH], ko[e], s[e]);
+        }
       }
-    }
-    if (active) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        if (!live[e]) continue;
-        const double val = w[e] == 1.0 ? s[e] + m[e] : fma(w[e], s[e], m[e]);
-        if (MODE == MODE_DU) {
-          A.du[(long)b * NV * S3 + (pidx[e] - (long)b * S3) + (NC + v) * S3] = val;
-        } else {
-          const long ai = (long)b * NV * S3 + (pidx[e] - (long)b * S3);
-          // the RK4 stage update of both halves of component v (EmitStage::fin)
-          if (A.stage == 4) {
-            A.next[wo[e] + v * sv] = fma(A.cb, kh[e], ah[e]);
-            A.next[wo[e] + (NC + v) * sv] = fma(A.cb, val, ap[e]);
+      if (!any) continue;
+      const double val0 = w[0] == 1.0 ? s[0] + m.x : fma(w[0], s[0], m.x);
+      const double val1 = w[1] == 1.0 ? s[1] + m.y : fma(w[1], s[1], m.y);
+      if (MODE == MODE_DU) {
+        if (live[0]) du[(NC + v) * S] = val0;
+        if (live[1]) du[(NC + v) * S + 1] = val1;
+      } else {
+        // the RK4 stage update of both halves of component v (EmitStage::fin)
+        auto put = [&](double* p, double x, double y) {
+          if (both) {
+            *reinterpret_cast<double2*>(p) = make_double2(x, y);
           } else {
-            A.acc[ai + v * S3] = fma(A.cb, kh[e], A.stage == 1 ? uh[e] : ah[e]);
-            A.acc[ai + (NC + v) * S3] = fma(A.cb, val, A.stage == 1 ? up[e] : ap[e]);
-            A.next[wo[e] + v * sv] = fma(A.ca, kh[e], uh[e]);
-            A.next[wo[e] + (NC + v) * sv] = fma(A.ca, val, up[e]);
+            if (live[0]) p[0] = x;
+            if (live[1]) p[1] = y;
           }
+        };
+        double* nh = A.next + wo + v * sv;
+        double* np = A.next + wo + (NC + v) * sv;
+        if (A.stage == 4) {
+          put(nh, fma(A.cb, kh.x, ah.x), fma(A.cb, kh.y, ah.y));
+          put(np, fma(A.cb, val0, ap.x), fma(A.cb, val1, ap.y));
+        } else {
+          const bool first = A.stage == 1;
+          put(acc + v * SX, fma(A.cb, kh.x, first ? uh.x : ah.x), fma(A.cb, kh.y, first ? uh.y : ah.y));
+          put(acc + (NC + v) * SX, fma(A.cb, val0, first ? up.x : ap.x), fma(A.cb, val1, first ? up.y : ap.y));
+          put(nh, fma(A.ca, kh.x, uh.x), fma(A.ca, kh.y, uh.y));
+          put(np, fma(A.ca, val0, up.x), fma(A.ca, val1, up.y));
         }
       }
     }
   }
   if (!ok) {
-    // a wait gave up: record it, let the copies already issued (component failed_at, and
-    // component 1 when it was the first) land, bounded, then leave without writing
+    // a wait gave up: record it, let the copies already issued (copy n, and copy 1 when n = 0)
+    // land, bounded, then leave without writing further
     if (tid == 0) atomicExch(stat.err, TGH_ERR_TIMEOUT);
     const long long drain = 1ll << 24;
-    const int last = failed_at == 0 ? 1 : failed_at;
-    for (int v = failed_at; v <= last; ++v) mbar_wait(v & 1 ? bar1 : bar0, (v >> 1) & 1, drain);
+    mbar_wait(bar0 + 8 * (n & 1), (n >> 1) & 1, drain);
+    if (n == 0) mbar_wait(bar0 + 8, 0, drain);
   }
 }
 

@@ -1,0 +1,50 @@
+// Tiled tensor copies into shared memory and the mbarriers they complete on, with bounded waits.
+#pragma once
+#include <cuda.h>
+
+namespace tgh {
+
+// The tensor maps of one working array, viewed as 4-d (x, y, z, block x 20 + variable): the Pi
+// kernel's boxes of h and Pi.
+struct TmaMaps {
+  CUtensorMap h, pi;
+};
+
+struct WaitStatus {
+  int* err;         // TGH_ERR_TIMEOUT is stored here by a wait that gives up
+  long long limit;  // polls a wait may make (negative: give up at once, which tests use)
+};
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded wait on one phase of an mbarrier: false when it gave up
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, long long limit) {
+  for (long long it = 0; it <= limit; ++it)
+    if (mbar_try_wait(bar, parity)) return true;
+  return false;
+}
+__device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map, int x, int y, int z, int c,
+                                            unsigned bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];" ::"r"(dst),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(c), "r"(bar)
+      : "memory");
+}
+
+}  // namespace tgh
