@@ -9,11 +9,9 @@
 // divergences and the source). With Phi = sum_v lambda_v du_v(p):
 //   * the features that enter linearly (the derivatives of Pi, the second derivatives of h, the
 //     dissipation of Pi) get their cotangents in closed form, coefficient x lambda;
-//   * the 50 nonlinear inputs - h (10), its first derivatives (30) and d_t h (10) - get theirs
-//     from 50 forward-mode passes of Phi in value-plus-derivative arithmetic (Tan), each seeding
-//     one input; d_t h's cotangent is passed on to Pi, the dissipation of h and, through the
-//     passes that seed h and its derivatives, the shift and lapse;
-//   * three more passes seed the parameters (rho_max, the ramp width, the damping strength).
+//   * the 50 nonlinear inputs - h (10), its first derivatives (30) and d_t h (10) - get theirs, and the
+//     parameters (rho_max, the ramp width, the damping strength) theirs, from one reverse sweep of the
+//     point's algebra (adjoint_algebra.cuh); d_t h's cotangent is passed on to Pi and the dissipation of h.
 // adjoint_gather_kernel then applies the transposed stencils: every point of the working array,
 // ghosts included, collects from the owned points whose stencils read it. The fill's transpose
 // follows (prolongation level by level from the finest, then the copies into the primary
@@ -22,6 +20,7 @@
 // 16 feature cotangents per component and point are kept, each feature a field in the padded
 // working layout (zero away from the owned points).
 #pragma once
+#include "adjoint_algebra.cuh"
 #include "kernels.cuh"
 #include "tangent_rhs.cuh"
 
@@ -30,7 +29,6 @@ namespace tgh {
 constexpr int ADJ_NF = 16;
 // per component: h value, dh (x,y,z), d2h (xx,yy,zz), mixed (xy,xz,yz), KO(h); Pi value, dPi (x,y,z), KO(Pi)
 enum { AF_HC = 0, AF_HD1 = 1, AF_HD2 = 4, AF_HMX = 7, AF_HKO = 10, AF_PC = 11, AF_PD1 = 12, AF_PKO = 15 };
-constexpr int ADJ_PASSES = 53;  // h (10), dh (30), d_t h (10), rho_max, ramp, damping
 
 struct AdjArgs {
   const double* lam;  // the cotangent of du, state layout
@@ -39,75 +37,9 @@ struct AdjArgs {
   double* part;       // 3 per CTA: the parameters' cotangents
 };
 
-// Phi along one seeded input (m < 10: h_m; m < 40: dh; m < 50: d_t h; 50..52: the parameters)
-template <bool DISS, bool INT>
-__device__ __forceinline__ Tan adjoint_phi(int m, const Case& cs, const RhsArgs& A, const PointIdx& q, double r, bool layer,
-                           const double* hv, const double* d1, const double* dth, const double* Pv,
-                           const double* koh, double eh, double ih, double ih2, const double* lh, const double* lP,
-                           const double* P1, double P0, const double* P2, double PKO, const double* he,
-                           const double* Pe) {
-  Tan hT[NC], dT[3][NC], dthT[NC];
-#pragma unroll
-  for (int v = 0; v < NC; ++v) hT[v] = Tan(hv[v], m == v ? 1.0 : 0.0);
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int v = 0; v < NC; ++v) dT[i][v] = Tan(d1[i * NC + v], m == NC + i * NC + v ? 1.0 : 0.0);
-  Coef<Tan> C;
-  metric_quantities(hT, C);
-  if (m >= 4 * NC && m < 5 * NC) {
-#pragma unroll
-    for (int v = 0; v < NC; ++v) dthT[v] = Tan(dth[v], m - 4 * NC == v ? 1.0 : 0.0);
-  } else {
-    const Tan adiv = C.alpha / C.sqrtg;
-#pragma unroll
-    for (int v = 0; v < NC; ++v) {
-      Tan s = C.beta[0] * dT[0][v] + C.beta[1] * dT[1][v] + C.beta[2] * dT[2][v] + adiv * Tan(Pv[v]);
-      if (DISS) s = fma(Tan(eh), Tan(koh[v]), s);
-      dthT[v] = s;
-    }
-  }
-  const int dir = m == 50 ? TAN_RHO_MAX : m == 51 ? TAN_RAMP : m == 52 ? TAN_DAMP_NEAR : TAN_STATE;
-  Tan wT = Tan(1.0), rhoT = Tan(0.0);
-  if (INT && layer) layer_profiles_t(cs, r, dir, wT, rhoT);
-  const Tan* dh[3] = {dT[0], dT[1], dT[2]};
-  Tan divb, divA[3];
-  metric_divergences(C, dh, divb, divA);
-  Tan msrc[NC];
-  const Tan* D[4] = {dthT, dT[0], dT[1], dT[2]};
-  rhs_source(cs, A, q.b, q.ip, damping_rate_t(cs, A.t, q.x, dir), hT, C, D, msrc);
-  // the Pi half: source + the stencil part contracted with the coefficients
-  Tan lin = C.beta[0] * Tan(ih * P1[0]) + C.beta[1] * Tan(ih * P1[1]) + C.beta[2] * Tan(ih * P1[2]) + divb * Tan(P0);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    Tan sd = Tan(0.0);
-#pragma unroll
-    for (int v = 0; v < NC; ++v) sd = fma(Tan(lP[v]), dT[i][v], sd);
-    lin = fma(divA[i], sd, lin);
-  }
-  const Tan am = C.alpha * C.sqrtg;
-  Tan a2 = am * C.gamu[0] * Tan(P2[0]) + am * C.gamu[3] * Tan(P2[1]) + am * C.gamu[5] * Tan(P2[2]);
-  a2 = a2 + Tan(2.0) * am * (C.gamu[1] * Tan(P2[3]) + C.gamu[2] * Tan(P2[4]) + C.gamu[4] * Tan(P2[5]));
-  lin = lin + Tan(ih2) * a2 + Tan(eh * PKO);
-  Tan phiP = lin;
-#pragma unroll
-  for (int v = 0; v < NC; ++v) phiP = fma(Tan(lP[v]), msrc[v], phiP);
-  Tan phi;
-  if (INT && layer) {
-    Tan relax = Tan(0.0);
-#pragma unroll
-    for (int v = 0; v < NC; ++v) relax = relax + Tan(lP[v] * (Pv[v] - Pe[v]));
-    phi = wT * phiP - rhoT * relax;
-#pragma unroll
-    for (int v = 0; v < NC; ++v) phi = phi + Tan(lh[v]) * (wT * dthT[v] - rhoT * (hT[v] - Tan(he[v])));
-  } else {
-    phi = phiP;
-#pragma unroll
-    for (int v = 0; v < NC; ++v) phi = fma(Tan(lh[v]), dthT[v], phi);
-  }
-  return phi;
-}
-
+// One thread per owned point. The algebra's working set (some 300 doubles) is in local memory, which the
+// L1 serves; 8 blocks of 16^3 take 0.28 ms (5.5 ms with the 53 forward passes this replaced, and 34 ms in the
+// instantiations whose registers the compiler then gave up on).
 template <int Q, bool DISS, bool INT>
 static __global__ void __launch_bounds__(128) adjoint_point_kernel(const Case cs, const RhsArgs A, const AdjArgs J) {
   __shared__ double sh[3][128];
@@ -189,28 +121,40 @@ static __global__ void __launch_bounds__(128) adjoint_point_kernel(const Case cs
         for (int i = 0; i < 3; ++i) cot(v, AF_HMX + i) = wl * ih2 * Ad[3 + i];
         cot(v, AF_PKO) = wl * eh;
       }
-      // the nonlinear inputs, one forward pass each
-      double g[ADJ_PASSES];
-#pragma unroll 1
-      for (int m = 0; m < ADJ_PASSES; ++m) {
-        if ((m == 50 || m == 51) && !layer) {
-          g[m] = 0.0;
-          continue;
+      // the nonlinear inputs, in one reverse sweep
+      double Hl[4], dHs[NC];
+      if (cs.gauge == TGH_GAUGE_SAMPLED) {
+        const double* hs = A.Hsrc + (long)q.b * NV * S + q.ip;  // rows: H_a (4), then d_c H_a at 4 + c + 4 a
+        for (int a = 0; a < 4; ++a) Hl[a] = hs[a * S];
+        for (int n = 0; n < NC; ++n) {
+          const int a = prow(n), c = pcol(n);
+          dHs[n] = hs[(4 + a + 4 * c) * S] + hs[(4 + c + 4 * a) * S];
         }
-        g[m] = adjoint_phi<DISS, INT>(m, cs, A, q, r, layer, hv, d1, dth, Pv, koh, eh, ih, ih2, lh, lP, P1, P0, P2,
-                                      PKO, he, Pe)
-                   .d;
       }
+      const Tan gd = damping_rate_t(cs, A.t, q.x, TAN_DAMP_NEAR);
+      PhiCotangents g;
+      adjoint_phi_reverse(cs, PhiInputs{hv, d1, dth, Pv, koh, eh, ih, ih2, lh, lP, P1, P2, P0, PKO, W, rho, gd.v, Hl, dHs},
+                          g);
       for (int v = 0; v < NC; ++v) {
-        cot(v, AF_HC) = g[v];
-        for (int i = 0; i < 3; ++i) cot(v, AF_HD1 + i) = g[NC + i * NC + v] * ih;
-        const double gd = g[4 * NC + v];
-        cot(v, AF_HKO) = gd * eh;
-        cot(v, AF_PC) = gd * adiv + W * lP[v] * divb - (layer ? rho * lP[v] : 0.0);
+        cot(v, AF_HC) = g.h[v];
+        for (int i = 0; i < 3; ++i) cot(v, AF_HD1 + i) = g.d1[i * NC + v] * ih;
+        cot(v, AF_HKO) = g.dth[v] * eh;
+        cot(v, AF_PC) = g.dth[v] * adiv + W * lP[v] * divb - rho * lP[v];
       }
-      th[0] = g[50];
-      th[1] = g[51];
-      th[2] = g[52];
+      if (INT && layer) {
+        // Phi = w (phiP + sum lh dth) - rho (sum lP (Pi - Pi_target) + sum lh (h - h_target))
+        double fw = g.phiP, fr = 0.0;
+        for (int v = 0; v < NC; ++v) {
+          fw = fma(lh[v], dth[v], fw);
+          fr = fma(lP[v], Pv[v] - Pe[v], fma(lh[v], hv[v] - he[v], fr));
+        }
+        for (int k = 0; k < 2; ++k) {
+          Tan wt, rt;
+          layer_profiles_t(cs, r, k == 0 ? TAN_RHO_MAX : TAN_RAMP, wt, rt);
+          th[k] = wt.d * fw - rt.d * fr;
+        }
+      }
+      th[2] = gd.d * g.g0;
     }
   }
   // the parameters' cotangents: per CTA, in a fixed order
