@@ -826,7 +826,7 @@ static int launch_interior(tgh_problem* p, const RhsArgs& a, int mode, cudaStrea
     L = &p->ilist;
   }
   if (L->n > 0) {
-    const long per = (p->S + 127) / 128;
+    const long per = (p->S + INTERIOR_CHUNK - 1) / INTERIOR_CHUNK;
     if (mode == MODE_DU)
       interior_kernel<MODE_DU><<<(unsigned)(L->n * per), 128, 0, s>>>(p->cs, a, L->dev);
     else
