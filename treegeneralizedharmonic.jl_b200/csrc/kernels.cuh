@@ -451,16 +451,31 @@ static __global__ void error_kernel(const double* __restrict__ work, const doubl
     part[3 * blockIdx.x + 2] = sh[2][0];
   }
 }
-static __global__ void error_final_kernel(const double* part, int n, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// The fold of the partials: each of the CTA's threads sums every 1024th in order, then a tree in a fixed
+// order (one thread for all of them took 1.9 ms for the 17,969 partials of 64 blocks of 32^3; this 9 us).
+static __global__ void __launch_bounds__(1024) error_final_kernel(const double* part, int n, double* out) {
+  __shared__ double sh[3][1024];
   double s2 = 0.0, vol = 0.0, mx = 0.0;
-  for (int i = 0; i < n; ++i) {
-    s2 += part[3 * i];
-    vol += part[3 * i + 1];
-    mx = fmax(mx, part[3 * i + 2]);
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    s2 += part[3 * (long)i];
+    vol += part[3 * (long)i + 1];
+    mx = fmax(mx, part[3 * (long)i + 2]);
   }
-  out[0] = vol == 0.0 ? 0.0 : sqrt(s2 / vol);
-  out[1] = mx;
+  sh[0][threadIdx.x] = s2;
+  sh[1][threadIdx.x] = vol;
+  sh[2][threadIdx.x] = mx;
+  __syncthreads();
+  for (int o = 512; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      sh[0][threadIdx.x] += sh[0][threadIdx.x + o];
+      sh[1][threadIdx.x] += sh[1][threadIdx.x + o];
+      sh[2][threadIdx.x] = fmax(sh[2][threadIdx.x], sh[2][threadIdx.x + o]);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return;
+  out[0] = sh[1][0] == 0.0 ? 0.0 : sqrt(sh[0][0] / sh[1][0]);
+  out[1] = sh[2][0];
 }
 
 // the case's state at every owned point (initial_state!); paste_only: only inside r_1 (the

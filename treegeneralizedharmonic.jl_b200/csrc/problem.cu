@@ -1641,7 +1641,7 @@ int tgh_error_norm(tgh_problem* p, const double* u, double t, double* l2, double
   if (s) return s;
   error_kernel<<<p->npart, 128, 0, p->stream>>>(p->work, p->blk, p->primary, p->geo, p->npts, p->cs, t, p->part);
   CK(cudaGetLastError());
-  error_final_kernel<<<1, 32, 0, p->stream>>>(p->part, p->npart, p->part + 3 * (size_t)p->npart);
+  error_final_kernel<<<1, 1024, 0, p->stream>>>(p->part, p->npart, p->part + 3 * (size_t)p->npart);
   CK(cudaGetLastError());
   double h[2];
   CK(cudaMemcpyAsync(h, p->part + 3 * (size_t)p->npart, sizeof(h), cudaMemcpyDeviceToHost, p->stream));
