@@ -204,6 +204,21 @@ static __global__ void transfer_copy_kernel(const CopyPt* __restrict__ pts, long
 #pragma unroll
   for (int v = 0; v < NV; ++v) dst[v * S] = src[v * g.Wv];
 }
+// the same for leaves that both forests have: block pairs (new, old), a thread per owned point. The old
+// array is filled, so the leaf's own copy of every point is the primary's value.
+static __global__ void transfer_block_kernel(const int2* __restrict__ pairs, int n, const double* __restrict__ work, Geo g,
+                                      double* __restrict__ u) {
+  const long id = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int S = (int)g.S, m = (int)(id / S);
+  if (m >= n) return;
+  const int2 pr = pairs[m];
+  const int ip = (int)(id - (long)m * S);
+  const int k = ip / (g.N1 * g.N1), j = (ip / g.N1) % g.N1, i = ip % g.N1;
+  const double* src = work + (long)pr.y * NV * g.Wv + work_index(g, i + g.G, j + g.G, k + g.G);
+  double* dst = u + (long)pr.x * NV * g.S + ip;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) dst[v * g.S] = src[v * g.Wv];
+}
 // one thread per (point, variable), consecutive threads on consecutive points of one variable:
 // their coarse stencils are neighbours in memory (the lists are grouped by odd-axis mask, so a
 // warp's points do the same amount of work)
