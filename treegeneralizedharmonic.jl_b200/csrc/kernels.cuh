@@ -608,14 +608,27 @@ static __global__ void sample_gauge_kernel(double* __restrict__ H, const double*
   for (int v = 0; v < NV; ++v) q[v * g.S] = v20[v];
 }
 
-// owned values of the working array back to the state vector (the batched form's output)
-static __global__ void gather_kernel(const double* __restrict__ work, double* __restrict__ u, Geo g, long npts) {
+// owned values of the working array back to the state vector (the batched form's output). With `beyond` (per
+// block the same-level leaf beyond its upper face along x, y, z, or -1) a point on a face that the batched form
+// left out is read where it was computed: on the lower face of that leaf, and on if it left the point out too.
+static __global__ void gather_kernel(const double* __restrict__ work, double* __restrict__ u, Geo g, long npts,
+                                     const int* __restrict__ beyond) {
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npts) return;
   const int b = (int)(p / g.S);
-  const long ip = p - (long)b * g.S;
-  const int k = (int)(ip / ((long)g.N1 * g.N1)), j = (int)((ip / g.N1) % g.N1), i = (int)(ip % g.N1);
-  const double* q = work + (long)b * NV * g.Wv + work_index(g, i + g.G, j + g.G, k + g.G);
+  const int ip = (int)(p - (long)b * g.S);
+  const int N = g.N1 - 1;
+  int s = b, k = ip / (g.N1 * g.N1), j = (ip / g.N1) % g.N1, i = ip % g.N1;
+  if (beyond) {
+    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0;
+    if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0;
+    if (k == N && beyond[3 * s + 2] >= 0) s = beyond[3 * s + 2], k = 0;
+    // the leaf reached along y or z may itself have a neighbour along x or y
+    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0;
+    if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0;
+    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0;
+  }
+  const double* q = work + (long)s * NV * g.Wv + work_index(g, i + g.G, j + g.G, k + g.G);
   double* o = u + (long)b * NV * g.S + ip;
 #pragma unroll
   for (int v = 0; v < NV; ++v) o[v * g.S] = q[v * g.Wv];

@@ -119,6 +119,12 @@ struct tgh_problem {
   int* ind_counts = nullptr;              // per block and threshold: firing count
   int* ind_boxes = nullptr;               // ... and the bounding box of the firing nodes
   double* coef = nullptr;                 // per-point coefficients between the two RHS kernels
+  // the batched form's computed points (RhsArgs): per block the same-level leaf beyond its upper faces whose lower
+  // face stands for them (or -1), the runs, the Pi kernel's tiles
+  int* beyond = nullptr;
+  PointRun* pruns = nullptr;
+  PiTile* ptiles = nullptr;
+  int npruns = 0, nptiles = 0;
   int npart = 0;
   // plain-form RK4 buffers (state layout)
   double *k = nullptr, *acc = nullptr, *y = nullptr, *u0 = nullptr;
@@ -479,6 +485,7 @@ static bool plan_rank(const tgh_problem* p, int r, bool entries, HostPlan& hp, s
 // to it, found by planning that rank's leaves: both sides derive the same sorted list).
 static bool tile_prolongation(const tgh_problem* p, const HostPlan& hp, const std::vector<ProlongPt>& pts,
                               std::vector<ProlongTile>& tiles, std::vector<unsigned short>& codes);
+static int build_computed(tgh_problem* p);
 static int build_plan(tgh_problem* p) {
   HostPlan hp;
   std::string err;
@@ -558,6 +565,58 @@ static int build_plan(tgh_problem* p) {
   }
   CK(cudaMalloc(&p->primary, (size_t)p->npts));
   CK(cudaMemcpy(p->primary, prim.data(), (size_t)p->npts, cudaMemcpyHostToDevice));
+  return build_computed(p);
+}
+
+// The points the batched form computes (RhsArgs' PointRun): per own block the same-level leaf of this rank beyond
+// each upper face, the runs of the remaining box and its Pi tiles. A face's copies are the same bits only if their
+// inputs are: across a periodic wrap the positions differ, so the wrap counts only where nothing depends on them.
+// A copy's source is computed: find_owner takes a level's leaf with the point on its lower faces first, so a
+// primary lies on an upper face only where no leaf of its level lies beyond it.
+static int build_computed(tgh_problem* p) {
+  const tgh_config& c = p->cfg;
+  const bool wraps = c.damping == TGH_DAMP_CONSTANT && c.dissipation == TGH_DISS_CONSTANT && !p->intr &&
+                     c.gauge == TGH_GAUGE_NONE;
+  std::vector<int> beyond(3 * (size_t)p->nb, -1);
+  for (int b = 0; b < p->nb; ++b) {
+    const int g = p->i2g[b], l = p->level[g];
+    for (int d = 0; d < 3; ++d) {
+      int64_t cn[3] = {p->corner[3 * g], p->corner[3 * g + 1], p->corner[3 * g + 2]};
+      cn[d] += p->N;
+      if (cn[d] == (int64_t)p->cells0[d] << l && p->periodic[d] && wraps) cn[d] = 0;
+      const auto it = p->lut[l].find(bkey(cn[0] / p->N, cn[1] / p->N, cn[2] / p->N));
+      if (it != p->lut[l].end() && p->owner[it->second] == p->rank) beyond[3 * b + d] = p->g2i[it->second];
+    }
+  }
+  std::vector<PointRun> runs;
+  std::vector<PiTile> tiles;
+  const bool tma = p->q == 4 && p->N == 32 && !p->mixed;
+  for (int b = 0; b < p->nb; ++b) {
+    int full = 0, n = 1, e[3];
+    for (int d = 0; d < 3; ++d) {
+      if (beyond[3 * b + d] < 0) full |= 1 << d;
+      e[d] = p->N + ((full >> d) & 1);
+      n *= e[d];
+    }
+    for (int m = 0; m < n; m += 128) runs.push_back(PointRun{b, m << 3 | full});
+    if (!tma) continue;
+    const bool inner = !(full & 3);
+    const int ty = inner ? pitma::Inner::TY : pitma::Whole::TY, tz = inner ? pitma::Inner::TZ : pitma::Whole::TZ;
+    for (int z = 0; z < e[2]; z += tz)
+      for (int y = 0; y < e[1]; y += ty)
+        tiles.push_back(PiTile{b, (unsigned char)y, (unsigned char)z,
+                               (unsigned char)(inner ? pitma::SHAPE_INNER : pitma::SHAPE_WHOLE), (unsigned char)full});
+  }
+  p->npruns = (int)runs.size();
+  p->nptiles = (int)tiles.size();
+  CK(cudaMalloc(&p->beyond, beyond.size() * sizeof(int)));
+  CK(cudaMemcpy(p->beyond, beyond.data(), beyond.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&p->pruns, runs.size() * sizeof(PointRun)));
+  CK(cudaMemcpy(p->pruns, runs.data(), runs.size() * sizeof(PointRun), cudaMemcpyHostToDevice));
+  if (!tiles.empty()) {
+    CK(cudaMalloc(&p->ptiles, tiles.size() * sizeof(PiTile)));
+    CK(cudaMemcpy(p->ptiles, tiles.data(), tiles.size() * sizeof(PiTile), cudaMemcpyHostToDevice));
+  }
   return TGH_OK;
 }
 
@@ -870,6 +929,10 @@ static RhsArgs base_args(tgh_problem* p, const double* work, double t) {
   a.p0 = 0;
   a.p1 = p->npts;
   a.t = t;
+  a.pruns = p->pruns;
+  a.npruns = p->npruns;
+  a.ptiles = p->ptiles;
+  a.nptiles = p->nptiles;
   a.threads = p->threads;
   a.pi_mb = p->pi_mb;
   return a;
@@ -1150,7 +1213,7 @@ void tgh_problem_destroy(tgh_problem* p) {
   }
   for (double* w : {p->work, p->W1, p->W2, p->twork})
     if (w) cudaFree(w - p->XO);
-  void* bufs[] = {p->Hsrc, p->tw, p->tf, p->blk, p->primary, p->runs, p->gpts, p->hooks, p->hook_cache, p->scratch,
+  void* bufs[] = {p->beyond, p->pruns, p->ptiles, p->Hsrc, p->tw, p->tf, p->blk, p->primary, p->runs, p->gpts, p->hooks, p->hook_cache, p->scratch,
                   p->bcounts, p->dev_err, p->ilist.dev, p->ilist_graph.dev,
                   p->part, p->coef, p->diag, p->dpart, p->ind, p->ind_tol, p->ind_counts, p->ind_boxes,
                   p->k, p->acc, p->y, p->u0, p->bacc, p->kt, p->acct, p->yt,
@@ -1527,7 +1590,7 @@ int tgh_gh_rhs(tgh_problem* p, double* du, const double* u, double t, const doub
 int tgh_settle(tgh_problem* p, double* u, double t) {
   int s = tgh_prepare(p, u, t);
   if (s) return s;
-  gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts);
+  gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts, nullptr);
   CK(cudaGetLastError());
   return TGH_OK;
 }
@@ -1918,7 +1981,7 @@ int tgh_step_batched(tgh_problem* p, double* u, double t, double dt, int nsteps)
     p->gkey = GraphKey{t, dt, nsteps};
   }
   CK(cudaGraphLaunch(p->gexec, p->stream));
-  gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts);
+  gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts, p->beyond);
   CK(cudaGetLastError());
   p->last_launches = fill_launches(p, false) + p->graph_kernels + 1;
   return TGH_OK;
@@ -2084,7 +2147,7 @@ int tgh_shard_rhs(tgh_problem* p, int stage, double t, double dt) {
 
 int tgh_shard_end(tgh_problem* p, double* u) {
   if (!p->W1) return fail(p, TGH_ERR_ARG, "tgh_shard_begin has not been called");
-  gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts);
+  gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts, p->beyond);
   CK(cudaGetLastError());
   p->last_launches = p->launches + 1;
   return TGH_OK;

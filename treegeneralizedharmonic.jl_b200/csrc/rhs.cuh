@@ -195,6 +195,22 @@ enum {
   NCOEF = CF_DTH0 + NC
 };
 
+// The batched form computes a point that several leaves of one level share once: a block leaves out its upper
+// face along an axis (i = N) where the leaf beyond it is of the same level and holds those points on its
+// lower face. Both copies have the same inputs (a ghost's value depends on its lattice point only), so they
+// would be the same bits; the stage fills overwrite the copy anyway, and the last gather reads the computed
+// one. Of 33^3 points a block that leaves 32^3 where all three neighbours exist, of 9^3 8^3.
+// The points of a block that are computed form a box of (N or N + 1)^3: `full` has a bit per axis that keeps
+// the upper face.
+struct PointRun {  // 128 consecutive points of a block's box from `start` on
+  int b;
+  int start_full;  // start << 3 | full
+};
+struct PiTile {    // a tile of rhs_pi_tma_kernel: its first row and plane, its shape
+  int b;
+  unsigned char y0, z0, shape, full;
+};
+
 // one launch's geometry and buffers
 struct RhsArgs {
   const double* work;     // ghosted working array, (W^3 x 20) per block
@@ -215,6 +231,10 @@ struct RhsArgs {
   long npts;              // N1^3 * nblocks
   long p0, p1;            // the points [p0, p1) this launch covers (whole blocks)
   double t;
+  // MODE_STAGE: the points the launch computes, as runs of 128 (PointRun), and the Pi kernel's tiles
+  const PointRun* pruns;
+  const PiTile* ptiles;
+  int npruns, nptiles;
   int threads;            // CTA size of the launch (64 or 128)
   int pi_mb;              // the one-point Pi kernel's resident CTAs per SM (3, 4 or 5)
 };
@@ -279,6 +299,25 @@ __device__ __forceinline__ PointIdx point_index(const RhsArgs& A, long p) {
   const int b = (int)(p / S);
   const int ip = (int)(p - (long)b * S);
   return point_at(A, b, ip % A.N1, (ip / A.N1) % A.N1, ip / (A.N1 * A.N1));
+}
+
+// the point of this thread in a launch of the head or one-point Pi kernel: of [p0, p1) in the plain form, of the
+// runs in the batched form
+template <int MODE> __device__ __forceinline__ bool launch_point(const RhsArgs& A, PointIdx& q) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (MODE == MODE_DU) {
+    if (A.p0 + t >= A.p1) return false;
+    q = point_index(A, A.p0 + t);
+    return true;
+  }
+  const PointRun r = A.pruns[t >> 7];
+  const int full = r.start_full & 7, N = A.N1 - 1;
+  const int ex = N + (full & 1), ey = N + ((full >> 1) & 1), ez = N + (full >> 2);
+  const int m = (r.start_full >> 3) + (int)(t & 127);
+  if (m >= ex * ey * ez) return false;
+  const int row = m / ex, k = row / ey;
+  q = point_at(A, r.b, m - row * ex, row - k * ey, k);
+  return true;
 }
 
 // The launch's geometry with the block size fixed at compile time when N1S > 0 (the usual
@@ -631,9 +670,8 @@ __global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsA
 template <int Q, bool DISS, int MODE, bool INT, int N1S, class T>
 __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(const Case cs, const RhsArgs A0) {
   const RhsArgs A = fixed_geometry<Q, N1S>(A0);
-  const long p = A.p0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= A.p1) return;
-  const PointIdx q = point_index(A, p);
+  PointIdx q;
+  if (!launch_point<MODE>(A, q)) return;
   const long S = (long)A.N1 * A.N1 * A.N1;
   const long sv = (long)A.Wx * A.Wd * A.Wd;
   const double* wk = A.work + q.wo;
@@ -715,9 +753,8 @@ __global__ void __launch_bounds__(128, is_fp32<T>() ? 3 : 1) rhs_head_kernel(con
 template <int Q, bool DISS, int MODE, class T, int N1S, int MB = 4>
 __global__ void __launch_bounds__(128, MB) rhs_pi_kernel(const Case cs, const RhsArgs A0) {
   const RhsArgs A = fixed_geometry<Q, N1S>(A0);
-  const long p = A.p0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= A.p1) return;
-  const PointIdx q = point_index(A, p);
+  PointIdx q;
+  if (!launch_point<MODE>(A, q)) return;
   const double* cfi = A.coef + q.cp;
   const double w = cfi[CF_W * A.ncoef];
   if (w < 0.0) return;

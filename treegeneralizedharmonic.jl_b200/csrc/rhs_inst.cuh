@@ -23,7 +23,8 @@ TGH_DECLARE_RHS_LAUNCH(8, f32)
 template <int Q, bool DISS, int MODE, int N1S, class T>
 cudaError_t launch_rhs_n(int part, bool intr, cudaStream_t s, const Case& cs, const RhsArgs& a) {
   const int TH = a.threads == 64 ? 64 : 128;
-  const unsigned nb = (unsigned)((a.p1 - a.p0 + TH - 1) / TH);
+  // the batched form's runs are of 128 points (a CTA of 64 takes half a run)
+  const unsigned nb = MODE == MODE_STAGE ? (unsigned)(a.npruns * (128 / TH)) : (unsigned)((a.p1 - a.p0 + TH - 1) / TH);
   if (part == 0) {
     if (intr) rhs_head_kernel<Q, DISS, MODE, true, N1S, T><<<nb, TH, 0, s>>>(cs, a);
     else rhs_head_kernel<Q, DISS, MODE, false, N1S, T><<<nb, TH, 0, s>>>(cs, a);

@@ -34,8 +34,10 @@ bool make_tma_maps(double* work, int nwb, TmaMaps* out, std::string& err) {
     return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, work, dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
-  CUresult r = map(&out->h, XB, Whole::HY, Whole::HZ);
-  if (r == CUDA_SUCCESS) r = map(&out->pi, XB, Whole::PY, Whole::PZ);
+  CUresult r = map(&out->whole.h, XB, Whole::HY, Whole::HZ);
+  if (r == CUDA_SUCCESS) r = map(&out->whole.pi, XB, Whole::PY, Whole::PZ);
+  if (r == CUDA_SUCCESS) r = map(&out->inner.h, XB, Inner::HY, Inner::HZ);
+  if (r == CUDA_SUCCESS) r = map(&out->inner.pi, XB, Inner::PY, Inner::PZ);
   if (r != CUDA_SUCCESS) {
     err = "cuTensorMapEncodeTiled refused the working array's map (error " + std::to_string((int)r) + ")";
     return false;
@@ -63,7 +65,7 @@ static cudaError_t launch_pi_tma_t(cudaStream_t s, const RhsArgs& a, const TmaMa
   int sms = 0;
   cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
-  const int tiles = nb * TILES;
+  const int tiles = MODE == MODE_STAGE ? a.nptiles : nb * TILES;
   rhs_pi_tma_kernel<DISS, MODE><<<(unsigned)(tiles < sms ? tiles : sms), THREADS, SMEM, s>>>(a, M, st, b0, tiles);
   return cudaGetLastError();
 }

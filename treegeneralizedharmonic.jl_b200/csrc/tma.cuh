@@ -4,10 +4,13 @@
 
 namespace tgh {
 
-// The tensor maps of one working array, viewed as 4-d (x, y, z, block x 20 + variable): the Pi
-// kernel's boxes of h and Pi.
-struct TmaMaps {
+// The tensor maps of one working array, viewed as 4-d (x, y, z, block x 20 + variable): the boxes of h and Pi
+// of the Pi kernel's two tile shapes.
+struct PiMaps {
   CUtensorMap h, pi;
+};
+struct TmaMaps {
+  PiMaps whole, inner;
 };
 
 struct WaitStatus {
