@@ -585,7 +585,9 @@ static int build_computed(tgh_problem* p) {
       cn[d] += p->N;
       if (cn[d] == (int64_t)p->cells0[d] << l && p->periodic[d] && wraps) cn[d] = 0;
       const auto it = p->lut[l].find(bkey(cn[0] / p->N, cn[1] / p->N, cn[2] / p->N));
-      if (it != p->lut[l].end() && p->owner[it->second] == p->rank) beyond[3 * b + d] = p->g2i[it->second];
+      // (a block alone on a periodic axis is not its own neighbour: its upper face is no copy the fill lists)
+      if (it != p->lut[l].end() && it->second != g && p->owner[it->second] == p->rank)
+        beyond[3 * b + d] = p->g2i[it->second];
     }
   }
   std::vector<PointRun> runs;
