@@ -85,6 +85,15 @@ TGH_HD RD operator/(const RD& a, const RD& b) {
   for (int i = 0; i < 4; ++i) r.d[i] = (a.d[i] * b.v - a.v * b.d[i]) / bb;
   return r;
 }
+// c a for a constant c: the product RD(c) * a without its products by the constant's zero partials, which are
+// zeros (for finite values) and change no sum
+TGH_HD RD rd_scale(double c, const RD& a) {
+  RD r;
+  r.v = RN(c) * a.v;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) r.d[i] = RN(c) * a.d[i];
+  return r;
+}
 TGH_HD RD rd_chain(const RD& a, RN f, RN df) {
   RD r;
   r.v = f;
@@ -102,36 +111,59 @@ TGH_HD RD rtanh_n(const RD& a) {
   return rd_chain(a, th, RN(1.0) - th * th);
 }
 
-// Kerr-Schild in its rest frame at (t, x, y, z): g = eta + 2 H l l
-TGH_HD void rn_kerr_schild(double M, double a, const RD x[4], RD g[4][4]) {
+// Kerr-Schild in its rest frame at (t, x, y, z), g = eta + 2 H l l: 2 H and l
+TGH_HD void rn_kerr_schild_lH(double M, double a, const RD x[4], RD& H2, RD l[4]) {
   const RD X = x[1], Y = x[2], Z = x[3];
   const RD rho2 = X * X + Y * Y + Z * Z;
-  const RD a2 = RD(a * a);
-  const RD half = RD(0.5) * (rho2 - a2);
-  const RD r2 = half + rsqrt_n(half * half + a2 * Z * Z);
+  const double a2 = TGH_RMUL(a, a);
+  RD half = rho2;
+  half.v = half.v - RN(a2);
+  half = rd_scale(0.5, half);
+  const RD a2Z2 = rd_scale(a2, Z) * Z;
+  const RD r2 = half + rsqrt_n(half * half + a2Z2);
   const RD r = rsqrt_n(r2);
-  const RD H = RD(M) * r * r2 / (r2 * r2 + a2 * Z * Z);
-  const RD den = r2 + a2;
-  const RD l[4] = {RD(1.0), (r * X + RD(a) * Y) / den, (r * Y - RD(a) * X) / den, Z / r};
+  H2 = rd_scale(2.0, rd_scale(M, r) * r2 / (r2 * r2 + a2Z2));
+  RD den = r2;
+  den.v = den.v + RN(a2);
+  l[0] = RD(1.0);
+  l[1] = (r * X + rd_scale(a, Y)) / den;
+  l[2] = (r * Y - rd_scale(a, X)) / den;
+  l[3] = Z / r;
+}
+// its component (i, j) from h = 2 H l_i
+TGH_HD RD rn_kerr_schild_ij(const RD& h, const RD l[4], int i, int j) {
+  RD e = h * l[j];
+  if (i == j) e.v = RN(etad(i)) + e.v;
+  return e;
+}
+TGH_HD void rn_kerr_schild(double M, double a, const RD x[4], RD g[4][4]) {
+  RD H2, l[4];
+  rn_kerr_schild_lH(M, a, x, H2, l);
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 4; ++i) {
+    const RD h = H2 * l[i];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) g[i][j] = RD(i == j ? etad(i) : 0.0) + RD(2.0) * H * l[i] * l[j];
+    for (int j = 0; j < 4; ++j) g[i][j] = rn_kerr_schild_ij(h, l, i, j);
+  }
 }
 
 // the rounded duals for the templated closed forms of physics.cuh (found by argument lookup)
 TGH_HD RD dsqrt(const RD& a) { return rsqrt_n(a); }
 TGH_HD void ks_rest(double M, double a, const RD* x, RD g[4][4]) { rn_kerr_schild(M, a, x, g); }
 
-// a hole's metric in its rest frame: Kerr-Schild, or Kerr in harmonic coordinates
-TGH_HD void rn_hole_rest(const Case& c, const RD x[4], RD g[4][4]) {
-  if (c.bg.kind == TGH_BG_HARMONIC_KERR)
-    harmonic_kerr_rest<RD>(c.bg.M, c.bg.a, x, g);
-  else
-    rn_kerr_schild(c.bg.M, c.bg.a, x, g);
+// the position in the boosted hole's rest frame
+TGH_HD void rn_boost(const Case& c, const RD x[4], RD xr[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    RD s = rd_scale(c.L[i][0], x[0]);
+#pragma unroll
+    for (int j = 1; j < 4; ++j) s = s + rd_scale(c.L[i][j], x[j]);
+    xr[i] = s;
+  }
 }
 
-// the case's metric g_ab with its first derivatives at xin = (t, x, y, z)
+// the case's metric g_ab with its first derivatives at xin = (t, x, y, z), every chart but the harmonic: at least the
+// components a >= b
 TGH_HD void rn_metric(const Case& c, const RD xin[4], RD g[4][4]) {
   RD x[4];
 #pragma unroll
@@ -150,33 +182,59 @@ TGH_HD void rn_metric(const Case& c, const RD xin[4], RD g[4][4]) {
     g[0][1] = -psi;
     g[1][0] = -psi;
     g[1][1] = RD(1.0) - psi * psi;
-  } else if (c.bg.kind == TGH_BG_KERR_SCHILD || c.bg.kind == TGH_BG_HARMONIC_KERR) {
+  } else if (c.bg.kind == TGH_BG_KERR_SCHILD) {
     if (!c.boosted) {
-      rn_hole_rest(c, x, g);
+      rn_kerr_schild(c.bg.M, c.bg.a, x, g);
       return;
     }
-    RD xr[4], gr[4][4];
+    // g_ab = sum_cd (L_ca L_db) g_rest_cd, c outer, d inner, with the sums of the ten components side by side, so
+    // that a rest-frame component lives only until it is added. Held as 16 duals beside the sums, and with the
+    // harmonic chart inlined beside them, an evaluation spilled 4 KB and was bound by that: the moving hole on
+    // 232 blocks takes 0.64 ms a stage for its interior (0.83) and 0.17 ms for its hook (0.22).
+    RD xr[4], H2, l[4], sm[NC];
+    rn_boost(c, x, xr);
+    rn_kerr_schild_lH(c.bg.M, c.bg.a, xr, H2, l);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      RD s = RD(c.L[i][0]) * x[0];
+    for (int n = 0; n < NC; ++n) sm[n] = RD(0.0);
 #pragma unroll
-      for (int j = 1; j < 4; ++j) s = s + RD(c.L[i][j]) * x[j];
-      xr[i] = s;
-    }
-    rn_hole_rest(c, xr, gr);
-    // g_ab = sum_cd (L_ca L_db) g_rest_cd, c outer, d inner
+    for (int p = 0; p < 4; ++p) {
+      const RD h = H2 * l[p];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+      for (int q = 0; q < 4; ++q) {
+        const RD e = rn_kerr_schild_ij(h, l, p, q);
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        RD s = RD(0.0);
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) s = s + RD(TGH_RMUL(c.L[p][a], c.L[q][b])) * gr[p][q];
-        g[a][b] = s;
+        for (int n = 0; n < NC; ++n) sm[n] = sm[n] + rd_scale(TGH_RMUL(c.L[p][prow(n)], c.L[q][pcol(n)]), e);
       }
+    }
+#pragma unroll
+    for (int n = 0; n < NC; ++n) g[prow(n)][pcol(n)] = sm[n];
   }
+}
+
+// the same for Kerr in harmonic coordinates. Called, not inlined: its duals fill the registers several times over,
+// and inlined beside the other charts they were spilled on every chart's path.
+static __host__ __device__ TGH_NOINLINE void rn_metric_harmonic(const Case& c, const RD xin[4], RD g[4][4]) {
+  RD x[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = xin[i] - RD(c.bg.translate[i]);
+  if (!c.boosted) {
+    harmonic_kerr_rest<RD>(c.bg.M, c.bg.a, x, g);
+    return;
+  }
+  RD xr[4], gr[4][4];
+  rn_boost(c, x, xr);
+  harmonic_kerr_rest<RD>(c.bg.M, c.bg.a, xr, gr);
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      RD s = RD(0.0);
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s = s + rd_scale(TGH_RMUL(c.L[p][a], c.L[q][b]), gr[p][q]);
+      g[a][b] = s;
+    }
 }
 
 TGH_HD RN rn_det3(RN a, RN b, RN c, RN d, RN e, RN f, RN g, RN h, RN i) {
@@ -294,7 +352,16 @@ static __host__ __device__ TGH_NOINLINE void rn_background_state(const Case& c, 
     p[i].d[i] = RN(1.0);
   }
   RD g[4][4];
-  rn_metric(c, p, g);
+  if (c.bg.kind == TGH_BG_HARMONIC_KERR) {
+    RD gh[4][4];
+    rn_metric_harmonic(c, p, gh);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) g[i][j] = gh[i][j];
+  } else {
+    rn_metric(c, p, g);
+  }
   RN hh[NC], dtg[NC], dh[3][NC];
 #pragma unroll
   for (int n = 0; n < NC; ++n) {
