@@ -225,6 +225,9 @@ int tgh_step_batched(tgh_problem* p, double* u, double t, double dt, int nsteps)
  *   pi_variant  TGH_PI_L1:  the Pi half as one point per thread, its stencils read through L1;
  *               TGH_PI_TMA: two points per thread from tiles of the working array staged into
  *               shared memory by the Tensor Memory Accelerator (q = 4, N = 32, FP64 only);
+ *               TGH_PI_TILE: the same scheme for every other FP64 problem with N <= 96, the tiles'
+ *               shape chosen for the block size and order, in the launches with enough points for it
+ *               to be the faster one (the one-point kernel in the others); the default there;
  *   threads     CTA size of the head and one-point Pi kernels, 64 or 128;
  *   pi_mb       the one-point Pi kernel's resident CTAs per SM (its launch bound), 3, 4 or 5.
  * All variants give the same bits. A change drops the batched form's captured graph.
@@ -232,7 +235,7 @@ int tgh_step_batched(tgh_problem* p, double* u, double t, double dt, int nsteps)
  * copies); a wait that runs out records TGH_ERR_TIMEOUT and its CTA writes nothing. A negative
  * limit gives up at once (for tests). tgh_device_status synchronizes the problem's stream and
  * returns (and clears) TGH_ERR_TIMEOUT if a wait gave up since the last call. */
-enum { TGH_PI_L1 = 0, TGH_PI_TMA = 1 };
+enum { TGH_PI_L1 = 0, TGH_PI_TMA = 1, TGH_PI_TILE = 2 };
 int tgh_set_variant(tgh_problem* p, int pi_variant, int threads, int pi_mb);
 int tgh_get_variant(const tgh_problem* p, int* pi_variant, int* threads, int* pi_mb);
 int tgh_set_wait_limit(tgh_problem* p, long long polls);

@@ -19,7 +19,7 @@ DISS_CONSTANT, DISS_HORIZON = range(2)
 INT_NONE, INT_DAMPED, INT_FROZEN, INT_PASTED, INT_FITTED = range(5)
 PREC_FP64, PREC_MIXED = range(2)
 MASK_INTERIOR, MASK_ALL = range(2)
-TGH_PI_L1, TGH_PI_TMA = range(2)
+TGH_PI_L1, TGH_PI_TMA, TGH_PI_TILE = range(3)
 NDIAG = 10  # diag slots per block: C_a (0..3), H (4), M_i (5..7), mask (8), tau (9)
 
 D3 = ctypes.c_double * 3

@@ -3,7 +3,8 @@
 The reference compiles its kernels per problem through KernelAbstractions and picks no launch
 shape itself. Here the choices are made by measurement on the GPU the problem runs on: for a
 problem (its mesh, order, precision and case), every candidate variant - the Pi half through L1
-at 3, 4 or 5 resident CTAs per SM or from TMA-staged tiles, the head and one-point Pi kernels at
+at 3, 4 or 5 resident CTAs per SM or from TMA-staged tiles ("tma" at q = 4 and N = 32, "tile" at the
+other sizes it serves), the head and one-point Pi kernels at
 64 or 128 threads a CTA - is timed over whole right-hand sides of the batched form (head + Pi,
 RK4 stage epilogue, CUDA events on the problem's stream), and the fastest is recorded in
 tuning/<gpu>.json under the configuration's key. GHProblem applies the recorded choice at
@@ -38,6 +39,9 @@ def candidates(problem):
     if problem.q == 4 and problem.forest.N == 32 and problem.precision == "fp64":
         for threads in (128, 64):
             out.append({"pi": "tma", "threads": threads, "pi_mb": 4})
+    elif problem.precision == "fp64" and 8 < problem.forest.N <= 96:
+        for threads in (128, 64):
+            out.append({"pi": "tile", "threads": threads, "pi_mb": 4})
     return out
 
 
@@ -84,6 +88,8 @@ def recorded_choice(problem, path=None):
     if not rec:
         return None
     choice = rec["choice"]
-    if choice["pi"] == "tma" and not (problem.q == 4 and problem.forest.N == 32 and problem.precision == "fp64"):
+    tma = problem.q == 4 and problem.forest.N == 32 and problem.precision == "fp64"
+    tile = not tma and problem.precision == "fp64" and problem.forest.N <= 96
+    if (choice["pi"] == "tma" and not tma) or (choice["pi"] == "tile" and not tile):
         return None
     return dict(choice)

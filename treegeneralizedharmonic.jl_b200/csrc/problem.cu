@@ -17,7 +17,7 @@
 #include "kernels.cuh"
 #include "monitors.cuh"
 #include "rhs_inst.cuh"
-#include "rhs_pi_tma.cuh"
+#include "rhs_pi_tile.cuh"
 #include "adjoint.cuh"
 #include "tangent_rhs.cuh"
 
@@ -25,6 +25,10 @@ using namespace tgh;
 
 namespace tgh {
 bool make_tma_maps(double* work, int nwb, TmaMaps* out, std::string& err);
+bool make_tile_maps(double* work, int nwb, int q, int N, const PiTileGeo& g, TmaMaps* out, std::string& err);
+bool pi_tile_geometry(int q, int N, int nwhole, int ninner, int sms, PiTileGeo* out);
+cudaError_t launch_pi_tile(int q, bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
+                           const PiTileGeo& g, int b0, int nb);
 cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
                           int b0, int nb);
 }  // namespace tgh
@@ -32,7 +36,7 @@ cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const RhsArgs& a,
 // the Pi kernel a problem launches: the one-point kernel reading through L1, or the pair kernel
 // whose stencil tiles the Tensor Memory Accelerator stages into shared memory (q = 4, N = 32,
 // FP64 only; the one-point kernel serves every other problem)
-enum { PI_L1 = TGH_PI_L1, PI_TMA = TGH_PI_TMA };
+enum { PI_L1 = TGH_PI_L1, PI_TMA = TGH_PI_TMA, PI_TILE = TGH_PI_TILE };
 
 struct GraphKey {
   double t, dt;
@@ -152,6 +156,7 @@ struct tgh_problem {
   // the right-hand side's kernel variants (tgh_set_variant) and the TMA kernel's tensor maps,
   // one pair per working array it has read
   int pi_variant = PI_L1;
+  PiTileGeo tile_geo{};  // the tile Pi kernel's geometry; threads = 0 where it does not apply
   int threads = 128;  // CTA size of the head and one-point Pi kernels
   int pi_mb = 4;      // the one-point Pi kernel's resident CTAs per SM (its launch bound)
   std::vector<std::pair<const double*, TmaMaps>> tma_maps;
@@ -593,6 +598,15 @@ static int build_computed(tgh_problem* p) {
   std::vector<PointRun> runs;
   std::vector<PiTile> tiles;
   const bool tma = p->q == 4 && p->N == 32 && !p->mixed;
+  if (!tma && !p->mixed) {
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int inner = 0;
+    for (int b = 0; b < p->nb; ++b) inner += beyond[3 * b] >= 0 && beyond[3 * b + 1] >= 0 && beyond[3 * b + 2] >= 0;
+    if (!pi_tile_geometry(p->q, p->N, p->nb - inner, inner, sms, &p->tile_geo)) p->tile_geo = PiTileGeo{};
+    if (p->tile_geo.threads) p->pi_variant = PI_TILE;
+  }
   for (int b = 0; b < p->nb; ++b) {
     int full = 0, n = 1, e[3];
     for (int d = 0; d < 3; ++d) {
@@ -601,9 +615,10 @@ static int build_computed(tgh_problem* p) {
       n *= e[d];
     }
     for (int m = 0; m < n; m += 128) runs.push_back(PointRun{b, m << 3 | full});
-    if (!tma) continue;
-    const bool inner = !(full & 3);
-    const int ty = inner ? pitma::Inner::TY : pitma::Whole::TY, tz = inner ? pitma::Inner::TZ : pitma::Whole::TZ;
+    if (!tma && !p->tile_geo.threads) continue;
+    const bool inner = tma ? !(full & 3) : full == 0;
+    const int ty = !tma ? p->tile_geo.shape[inner].TY : inner ? pitma::Inner::TY : pitma::Whole::TY;
+    const int tz = !tma ? p->tile_geo.shape[inner].TZ : inner ? pitma::Inner::TZ : pitma::Whole::TZ;
     for (int z = 0; z < e[2]; z += tz)
       for (int y = 0; y < e[1]; y += ty)
         tiles.push_back(PiTile{b, (unsigned char)y, (unsigned char)z,
@@ -818,13 +833,28 @@ static bool tma_applies(const tgh_problem* p, const RhsArgs& a) {
   return p->pi_variant == PI_TMA && p->q == 4 && p->N == 32 && !p->mixed && a.p0 % p->S == 0 && a.p1 % p->S == 0;
 }
 
+// Whether a launch takes the tile Pi kernel: the variant chosen, whole blocks, and enough points to fill the GPU with
+// tiles. Where the line lies (us a right-hand side, one-point against tile): at q >= 4 in the plain form 8 blocks of
+// 12^3 (17,576 points) 37 against 54 and of 16^3 (39,304) 52 against 44; in the batched form, whose epilogue both
+// wait for, 8 of 16^3 46 against 47 (q = 4) and 42 against 46 (q = 6), 64 of 16^3 (262,144 computed) 269 against 208
+// and 267 against 253; the batched form's rows of 8 points share banks, 2472 blocks of 8^3 1,582 against 1,584. At
+// q = 2 there is less to share: 8 blocks of 32^3 121 against 131, 27 of 27^3 333 against 269.
+static bool tile_applies(const tgh_problem* p, const RhsArgs& a, int mode) {
+  if (p->pi_variant != PI_TILE || a.p0 % p->S != 0 || a.p1 % p->S != 0) return false;
+  const long points = mode == MODE_STAGE ? 128L * a.npruns : a.p1 - a.p0;
+  if (p->q == 2) return points >= 500000;
+  return mode == MODE_STAGE ? points >= 100000 && p->N > 8 : points >= 32768;
+}
+
 // the tensor maps of one of the problem's working arrays (made once per array)
 static const TmaMaps* work_tma_maps(tgh_problem* p, const double* work) {
   for (auto& e : p->tma_maps)
     if (e.first == work) return &e.second;
   TmaMaps m;
   std::string err;
-  if (!make_tma_maps(const_cast<double*>(work) - p->XO, p->nwb, &m, err)) {
+  double* base = const_cast<double*>(work) - p->XO;
+  if (!(p->tile_geo.threads ? make_tile_maps(base, p->nwb, p->q, p->N, p->tile_geo, &m, err)
+                       : make_tma_maps(base, p->nwb, &m, err))) {
     p->err = err;
     return nullptr;
   }
@@ -908,6 +938,13 @@ static int launch_rhs(tgh_problem* p, const RhsArgs& a, int mode) {
     if (!M) return TGH_ERR_CUDA;
     CK(launch_pi_tma(p->diss, mode, p->stream, a, *M, WaitStatus{p->dev_err, p->wait_limit}, (int)(a.p0 / p->S),
                      (int)((a.p1 - a.p0) / p->S)));
+    return TGH_OK;
+  }
+  if (tile_applies(p, a, mode)) {
+    const TmaMaps* M = work_tma_maps(p, a.work);
+    if (!M) return TGH_ERR_CUDA;
+    CK(launch_pi_tile(p->q, p->diss, mode, p->stream, a, *M, WaitStatus{p->dev_err, p->wait_limit}, p->tile_geo,
+                      (int)(a.p0 / p->S), (int)((a.p1 - a.p0) / p->S)));
     return TGH_OK;
   }
   CK(launch_part(p, 1, mode, p->stream, a));
@@ -1529,12 +1566,15 @@ int tgh_copy_diag(tgh_problem* p, double* out) {
 
 // ---- the right-hand side's kernel variants (the autotuner's choices) and device waits ----
 int tgh_set_variant(tgh_problem* p, int pi_variant, int threads, int pi_mb) {
-  if (pi_variant != TGH_PI_L1 && pi_variant != TGH_PI_TMA) return fail(p, TGH_ERR_ARG, "unknown Pi kernel variant");
+  if (pi_variant != TGH_PI_L1 && pi_variant != TGH_PI_TMA && pi_variant != TGH_PI_TILE)
+    return fail(p, TGH_ERR_ARG, "unknown Pi kernel variant");
+  if (pi_variant == TGH_PI_TILE && !p->tile_geo.threads)
+    return fail(p, TGH_ERR_ARG, "the tile Pi kernel serves FP64 problems that the TMA Pi kernel does not, N <= 96");
   if (pi_variant == TGH_PI_TMA && !(p->q == 4 && p->N == 32 && !p->mixed))
     return fail(p, TGH_ERR_ARG, "the TMA Pi kernel serves q = 4, N = 32, FP64 problems only");
   if (threads != 64 && threads != 128) return fail(p, TGH_ERR_ARG, "the CTA size must be 64 or 128");
   if (pi_mb < 3 || pi_mb > 5) return fail(p, TGH_ERR_ARG, "the one-point Pi kernel's CTAs per SM must be 3, 4 or 5");
-  if (pi_variant == TGH_PI_TMA) {
+  if (pi_variant != TGH_PI_L1) {
     // check now that the driver can describe the working array to the copy engine
     if (!work_tma_maps(p, p->work)) return TGH_ERR_CUDA;
   }

@@ -1,0 +1,6 @@
+// The tile Pi kernel's instantiations for finite-difference order q = 2.
+#include "rhs_pi_tile.cuh"
+
+namespace tgh {
+TGH_DEFINE_PI_TILE(2)
+}  // namespace tgh

@@ -5,7 +5,7 @@
 namespace tgh {
 
 // The tensor maps of one working array, viewed as 4-d (x, y, z, block x 20 + variable): the boxes of h and Pi
-// of the Pi kernel's two tile shapes.
+// of the TMA Pi kernel's two tile shapes, or of the tile Pi kernel's (whole).
 struct PiMaps {
   CUtensorMap h, pi;
 };

@@ -87,12 +87,12 @@ class GHProblem:
         self._check(self.lib.tgh_rhs(self._h, _ptr(du), float(t), _ptr(matter)))
 
     # ---- the right-hand side's kernel variants (tgh_set_variant) ----
-    PI_VARIANTS = {"l1": _abi.TGH_PI_L1, "tma": _abi.TGH_PI_TMA}
+    PI_VARIANTS = {"l1": _abi.TGH_PI_L1, "tma": _abi.TGH_PI_TMA, "tile": _abi.TGH_PI_TILE}
 
     def set_variant(self, pi="l1", threads=128, pi_mb=4):
         """The kernels the right-hand side launches: the Pi half through L1 ("l1") or from tiles
-        staged by the Tensor Memory Accelerator ("tma", q = 4 and N = 32 only), the CTA size of
-        the head and one-point Pi kernels, the one-point Pi kernel's resident CTAs per SM."""
+        staged by the Tensor Memory Accelerator ("tma": q = 4 and N = 32; "tile": the other FP64
+        problems), the CTA size of the head and one-point Pi kernels, the one-point Pi kernel's resident CTAs per SM."""
         self._check(self.lib.tgh_set_variant(self._h, self.PI_VARIANTS[pi], int(threads), int(pi_mb)))
 
     def variant(self):
