@@ -620,13 +620,14 @@ static __global__ void gather_kernel(const double* __restrict__ work, double* __
   const int N = g.N1 - 1;
   int s = b, k = ip / (g.N1 * g.N1), j = (ip / g.N1) % g.N1, i = ip % g.N1;
   if (beyond) {
-    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0;
-    if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0;
-    if (k == N && beyond[3 * s + 2] >= 0) s = beyond[3 * s + 2], k = 0;
-    // the leaf reached along y or z may itself have a neighbour along x or y
-    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0;
-    if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0;
-    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0;
+    // until no move applies: the leaf a move reaches may leave the point out along an axis tried before. A move takes
+    // its axis off the upper face, so there are three at most.
+    for (bool moved = true; moved;) {
+      moved = false;
+      if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0, moved = true;
+      if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0, moved = true;
+      if (k == N && beyond[3 * s + 2] >= 0) s = beyond[3 * s + 2], k = 0, moved = true;
+    }
   }
   const double* q = work + (long)s * NV * g.Wv + work_index(g, i + g.G, j + g.G, k + g.G);
   double* o = u + (long)b * NV * g.S + ip;
