@@ -129,7 +129,8 @@ def computed_points(case, forest, owner=None):
     upper face where another leaf of its level (of its rank) lies beyond. A periodic wrap counts only where nothing
     depends on the position."""
     N = forest.N
-    wraps = not (case.interior or isinstance(case.gamma0, dict) or isinstance(case.eps_ko, dict) or case.gauge != "none")
+    wraps = all(forest.periodic) and not (case.interior or isinstance(case.gamma0, dict) or
+                                          isinstance(case.eps_ko, dict) or case.gauge != "none")
     own = owner if owner is not None else [0] * forest.nblocks
     leaves = {(int(l), tuple(int(x) // N for x in c)): int(o) for l, c, o in zip(forest.level, forest.corner, own)}
     total = 0

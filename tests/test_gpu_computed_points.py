@@ -1,8 +1,9 @@
 """The batched form computes a point that same-level leaves share once (RhsArgs' PointRun) and reads it back
 for every copy: the plain form, which computes every copy, gives the same bits - on one periodic block that is
 its own neighbour, on meshes whose blocks keep all, some or none of their upper faces, with odd edges, and
-across refinement faces, where a face stays when the leaf beyond is of another level, and around a vertex
-whose computed copy is three moves away in only one order of the axes."""
+across refinement faces, where a face stays when the leaf beyond is of another level, around a vertex whose
+computed copy is three moves away in only one order of the axes, and across a periodic wrap beside a Dirichlet
+boundary, whose values differ by rounding between the two faces."""
 from dataclasses import replace
 
 import numpy as np
@@ -29,8 +30,9 @@ def refined_roots(tgh, case, N, refined):
                       np.array([c for _, c in leaves], dtype=np.int32))
 
 
-def wave(tgh, periodic):
-    return replace(tgh.gauge_wave_case(eps_ko=0.5, gamma0=1.0), periodic=periodic)
+def wave(tgh, periodic, A=0.05, d=1.0):
+    return replace(tgh.gauge_wave_case(A=A, eps_ko=0.5, gamma0=1.0), background={"kind": "gauge_wave", "A": A, "d": d},
+                   periodic=periodic)
 
 
 # the same-level leaves around the centre are (0, 0, 0), (0, 1, 0), (1, 1, 0), (1, 1, 1) and an axis permutation of
@@ -52,6 +54,7 @@ MESHES = {
                                     lambda c: t.hole_forest(c, 32, 2, [1.6]), 4),
     **{f"stairs_{k}": lambda t, r=r: (wave(t, (False,) * 3), lambda c: refined_roots(t, c, 8, r), 4)
        for k, r in STAIRS.items()},
+    "wrap_beside_dirichlet": lambda t: (wave(t, (True, False, True), 0.4, 1 / 3), lambda c: t.gh_forest(c, 8, 2), 4),
 }
 
 

@@ -575,13 +575,14 @@ static int build_plan(tgh_problem* p) {
 
 // The points the batched form computes (RhsArgs' PointRun): per own block the same-level leaf of this rank beyond
 // each upper face, the runs of the remaining box and its Pi tiles. A face's copies are the same bits only if their
-// inputs are: across a periodic wrap the positions differ, so the wrap counts only where nothing depends on them.
+// inputs are: across a periodic wrap the positions differ, so the wrap counts only where nothing depends on them,
+// the ghosts beyond a Dirichlet boundary included (each copy's are the state at its own side of the wrap).
 // A copy's source is computed: find_owner takes a level's leaf with the point on its lower faces first, so a
 // primary lies on an upper face only where no leaf of its level lies beyond it.
 static int build_computed(tgh_problem* p) {
   const tgh_config& c = p->cfg;
   const bool wraps = c.damping == TGH_DAMP_CONSTANT && c.dissipation == TGH_DISS_CONSTANT && !p->intr &&
-                     c.gauge == TGH_GAUGE_NONE;
+                     c.gauge == TGH_GAUGE_NONE && p->periodic[0] && p->periodic[1] && p->periodic[2];
   std::vector<int> beyond(3 * (size_t)p->nb, -1);
   for (int b = 0; b < p->nb; ++b) {
     const int g = p->i2g[b], l = p->level[g];
