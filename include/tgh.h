@@ -159,7 +159,8 @@ size_t tgh_work_length(const tgh_problem* p);
  * from their primary, owned copies that are not primary), [1] Dirichlet ghosts, [2] prolonged
  * points of all levels, [3] prolongation tiles (0 where a level runs point by point) */
 int tgh_fill_counts(const tgh_problem* p, long long counts[4]);
-/* copy the working array (device to device) for inspection */
+/* copy the working array (device to device) for inspection: after tgh_prepare that fill, after a batched step the
+ * state at every owned point (the ghosts are then the last stage's leftovers) */
 int tgh_copy_work(tgh_problem* p, double* dst);
 /* the same for the blocks b0 .. b0 + nblocks - 1 of the working array (each (N+2G+1)^3 * 20
  * doubles, blocks in forest order on a problem of one rank) */

@@ -608,31 +608,47 @@ static __global__ void sample_gauge_kernel(double* __restrict__ H, const double*
   for (int v = 0; v < NV; ++v) q[v * g.S] = v20[v];
 }
 
-// owned values of the working array back to the state vector (the batched form's output). With `beyond` (per
-// block the same-level leaf beyond its upper face along x, y, z, or -1) a point on a face that the batched form
-// left out is read where it was computed: on the lower face of that leaf, and on if it left the point out too.
+// The copy of the owned point (i, j, k) of block s that the batched form computed. With `beyond` (per block the
+// same-level leaf beyond its upper face along x, y, z, or -1) a point on a face that was left out is computed on the
+// lower face of that leaf, and on if it left the point out too: until no move applies, as the leaf a move reaches may
+// leave the point out along an axis tried before. A move takes its axis off the upper face, so there are three at most.
+__device__ __forceinline__ void computed_copy(const int* __restrict__ beyond, int N, int& s, int& i, int& j, int& k) {
+  for (bool moved = true; moved;) {
+    moved = false;
+    if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0, moved = true;
+    if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0, moved = true;
+    if (k == N && beyond[3 * s + 2] >= 0) s = beyond[3 * s + 2], k = 0, moved = true;
+  }
+}
+// owned values of the working array back to the state vector (the batched form's output, with `beyond`)
 static __global__ void gather_kernel(const double* __restrict__ work, double* __restrict__ u, Geo g, long npts,
                                      const int* __restrict__ beyond) {
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npts) return;
   const int b = (int)(p / g.S);
   const int ip = (int)(p - (long)b * g.S);
-  const int N = g.N1 - 1;
   int s = b, k = ip / (g.N1 * g.N1), j = (ip / g.N1) % g.N1, i = ip % g.N1;
-  if (beyond) {
-    // until no move applies: the leaf a move reaches may leave the point out along an axis tried before. A move takes
-    // its axis off the upper face, so there are three at most.
-    for (bool moved = true; moved;) {
-      moved = false;
-      if (i == N && beyond[3 * s] >= 0) s = beyond[3 * s], i = 0, moved = true;
-      if (j == N && beyond[3 * s + 1] >= 0) s = beyond[3 * s + 1], j = 0, moved = true;
-      if (k == N && beyond[3 * s + 2] >= 0) s = beyond[3 * s + 2], k = 0, moved = true;
-    }
-  }
+  if (beyond) computed_copy(beyond, g.N1 - 1, s, i, j, k);
   const double* q = work + (long)s * NV * g.Wv + work_index(g, i + g.G, j + g.G, k + g.G);
   double* o = u + (long)b * NV * g.S + ip;
 #pragma unroll
   for (int v = 0; v < NV; ++v) o[v * g.S] = q[v * g.Wv];
+}
+// the points a batched step left out, in its working array: each from the copy that was computed. None of those is
+// left out itself, so no thread reads what another writes; after a fill the copies agree and nothing changes.
+static __global__ void complete_kernel(double* work, Geo g, long npts, const int* __restrict__ beyond) {
+  const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= npts) return;
+  const int b = (int)(p / g.S);
+  const int ip = (int)(p - (long)b * g.S);
+  const int k = ip / (g.N1 * g.N1), j = (ip / g.N1) % g.N1, i = ip % g.N1;
+  int s = b, si = i, sj = j, sk = k;
+  computed_copy(beyond, g.N1 - 1, s, si, sj, sk);
+  if (s == b) return;
+  const double* q = work + (long)s * NV * g.Wv + work_index(g, si + g.G, sj + g.G, sk + g.G);
+  double* o = work + (long)b * NV * g.Wv + work_index(g, i + g.G, j + g.G, k + g.G);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) o[v * g.Wv] = q[v * g.Wv];
 }
 
 // the owned points of the first npts / S blocks of a working array from the state vector u

@@ -1283,7 +1283,7 @@ int tgh_fill_counts(const tgh_problem* p, long long counts[4]) {
   return TGH_OK;
 }
 // The ABI's view of the working array is the reference's layout, (N+2G+1)^3 points per block
-// and variable; the problem stores rows padded to the even pitch Wx.
+// and variable; the problem stores rows padded to the pitch Wx (row_pitch).
 size_t tgh_work_length(const tgh_problem* p) { return (size_t)p->Wd * p->Wd * p->Wd * NV * p->nwb; }
 
 int tgh_copy_work(tgh_problem* p, double* dst) { return tgh_copy_work_blocks(p, 0, p->nwb, dst); }
@@ -1291,6 +1291,10 @@ int tgh_copy_work(tgh_problem* p, double* dst) { return tgh_copy_work_blocks(p, 
 int tgh_copy_work_blocks(tgh_problem* p, int b0, int nblocks, double* dst) {
   if (b0 < 0 || nblocks < 0 || b0 + nblocks > p->nwb) return fail(p, TGH_ERR_ARG, "block range out of bounds");
   if (nblocks == 0) return TGH_OK;
+  // after a batched step the points it left out still hold what they held before it: the array shows the state at
+  // every owned point
+  complete_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, p->geo, p->npts, p->beyond);
+  CK(cudaGetLastError());
   // one row of Wd doubles per copy: rows of the padded array are Wx apart, of the dense one Wd
   const size_t rows = (size_t)p->Wd * p->Wd * NV * nblocks;
   CK(cudaMemcpy2DAsync(dst, (size_t)p->Wd * sizeof(double), p->work + (size_t)p->Wv * NV * b0,
