@@ -28,9 +28,9 @@ bool make_tma_maps(double* work, int nwb, TmaMaps* out, std::string& err);
 bool make_tile_maps(double* work, int nwb, int q, int N, const PiTileGeo& g, TmaMaps* out, std::string& err);
 bool pi_tile_geometry(int q, int N, int nwhole, int ninner, int sms, PiTileGeo* out);
 cudaError_t launch_pi_tile(int q, bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
-                           const PiTileGeo& g, int b0, int nb);
+                           const PiTileGeo& g, const PiLaunch& L);
 cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
-                          int b0, int nb);
+                          const PiLaunch& L);
 }  // namespace tgh
 
 // the Pi kernel a problem launches: the one-point kernel reading through L1, or the pair kernel
@@ -157,6 +157,8 @@ struct tgh_problem {
   // one pair per working array it has read
   int pi_variant = PI_L1;
   PiTileGeo tile_geo{};  // the tile Pi kernel's geometry; threads = 0 where it does not apply
+  int sms = 0;        // of the problem's device
+  bool pi_launched[2] = {false, false};  // whether a staged Pi kernel was launched in a form (PiLaunch::first)
   int threads = 128;  // CTA size of the head and one-point Pi kernels
   int pi_mb = 4;      // the one-point Pi kernel's resident CTAs per SM (its launch bound)
   std::vector<std::pair<const double*, TmaMaps>> tma_maps;
@@ -599,13 +601,13 @@ static int build_computed(tgh_problem* p) {
   std::vector<PointRun> runs;
   std::vector<PiTile> tiles;
   const bool tma = p->q == 4 && p->N == 32 && !p->mixed;
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
   if (!tma && !p->mixed) {
-    int dev = 0, sms = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int inner = 0;
     for (int b = 0; b < p->nb; ++b) inner += beyond[3 * b] >= 0 && beyond[3 * b + 1] >= 0 && beyond[3 * b + 2] >= 0;
-    if (!pi_tile_geometry(p->q, p->N, p->nb - inner, inner, sms, &p->tile_geo)) p->tile_geo = PiTileGeo{};
+    if (!pi_tile_geometry(p->q, p->N, p->nb - inner, inner, p->sms, &p->tile_geo)) p->tile_geo = PiTileGeo{};
     if (p->tile_geo.threads) p->pi_variant = PI_TILE;
   }
   for (int b = 0; b < p->nb; ++b) {
@@ -934,18 +936,16 @@ static int launch_rhs(tgh_problem* p, const RhsArgs& a, int mode) {
     if (s) return s;
   }
   CK(launch_part(p, 0, mode, p->stream, a));
-  if (tma_applies(p, a)) {
+  const bool tma = tma_applies(p, a);
+  if (tma || tile_applies(p, a, mode)) {
     const TmaMaps* M = work_tma_maps(p, a.work);
     if (!M) return TGH_ERR_CUDA;
-    CK(launch_pi_tma(p->diss, mode, p->stream, a, *M, WaitStatus{p->dev_err, p->wait_limit}, (int)(a.p0 / p->S),
-                     (int)((a.p1 - a.p0) / p->S)));
-    return TGH_OK;
-  }
-  if (tile_applies(p, a, mode)) {
-    const TmaMaps* M = work_tma_maps(p, a.work);
-    if (!M) return TGH_ERR_CUDA;
-    CK(launch_pi_tile(p->q, p->diss, mode, p->stream, a, *M, WaitStatus{p->dev_err, p->wait_limit}, p->tile_geo,
-                      (int)(a.p0 / p->S), (int)((a.p1 - a.p0) / p->S)));
+    bool& launched = p->pi_launched[mode == MODE_STAGE];
+    const PiLaunch L{(int)(a.p0 / p->S), (int)((a.p1 - a.p0) / p->S), p->sms, !launched};
+    const WaitStatus st{p->dev_err, p->wait_limit};
+    CK(tma ? launch_pi_tma(p->diss, mode, p->stream, a, *M, st, L)
+           : launch_pi_tile(p->q, p->diss, mode, p->stream, a, *M, st, p->tile_geo, L));
+    launched = true;
     return TGH_OK;
   }
   CK(launch_part(p, 1, mode, p->stream, a));

@@ -36,7 +36,7 @@ constexpr int PI_TILE_SMEM = 227 * 1024;  // one CTA an SM
 
 #define TGH_DECLARE_PI_TILE(QQ)                                                                                   \
   cudaError_t launch_pi_tile_q##QQ(bool diss, int mode, unsigned grid, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, \
-                                   WaitStatus st, const PiTileGeo& g, int b0, int tiles);
+                                   WaitStatus st, const PiTileGeo& g, const PiLaunch& L, int tiles);
 TGH_DECLARE_PI_TILE(2)
 TGH_DECLARE_PI_TILE(4)
 TGH_DECLARE_PI_TILE(6)
@@ -410,21 +410,22 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
 
 template <int Q, bool DISS, int MODE>
 cudaError_t launch_pi_tile_t(unsigned grid, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
-                             const PiTileGeo& g, int b0, int tiles) {
-  // every call, since the attribute is per device
-  const cudaError_t e = cudaFuncSetAttribute(rhs_pi_tile_kernel<Q, DISS, MODE>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, PI_TILE_SMEM);
-  if (e != cudaSuccess) return e;
-  rhs_pi_tile_kernel<Q, DISS, MODE><<<grid, g.threads, g.smem, s>>>(a, M, st, g, b0, tiles);
+                             const PiTileGeo& g, const PiLaunch& L, int tiles) {
+  if (L.first) {
+    const cudaError_t e = cudaFuncSetAttribute(rhs_pi_tile_kernel<Q, DISS, MODE>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, PI_TILE_SMEM);
+    if (e != cudaSuccess) return e;
+  }
+  rhs_pi_tile_kernel<Q, DISS, MODE><<<grid, g.threads, g.smem, s>>>(a, M, st, g, L.b0, tiles);
   return cudaGetLastError();
 }
 #define TGH_DEFINE_PI_TILE(QQ)                                                                                    \
   cudaError_t launch_pi_tile_q##QQ(bool diss, int mode, unsigned grid, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, \
-                                   WaitStatus st, const PiTileGeo& g, int b0, int tiles) {                        \
-    if (diss) return mode == MODE_DU ? launch_pi_tile_t<QQ, true, MODE_DU>(grid, s, a, M, st, g, b0, tiles)                     \
-                                     : launch_pi_tile_t<QQ, true, MODE_STAGE>(grid, s, a, M, st, g, b0, tiles);                 \
-    return mode == MODE_DU ? launch_pi_tile_t<QQ, false, MODE_DU>(grid, s, a, M, st, g, b0, tiles)                              \
-                           : launch_pi_tile_t<QQ, false, MODE_STAGE>(grid, s, a, M, st, g, b0, tiles);                          \
+                                   WaitStatus st, const PiTileGeo& g, const PiLaunch& L, int tiles) {             \
+    if (diss) return mode == MODE_DU ? launch_pi_tile_t<QQ, true, MODE_DU>(grid, s, a, M, st, g, L, tiles)                      \
+                                     : launch_pi_tile_t<QQ, true, MODE_STAGE>(grid, s, a, M, st, g, L, tiles) ;                 \
+    return mode == MODE_DU ? launch_pi_tile_t<QQ, false, MODE_DU>(grid, s, a, M, st, g, L, tiles)                               \
+                           : launch_pi_tile_t<QQ, false, MODE_STAGE>(grid, s, a, M, st, g, L, tiles) ;                          \
   }
 
 }  // namespace tgh

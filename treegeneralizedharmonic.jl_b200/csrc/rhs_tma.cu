@@ -125,53 +125,38 @@ bool pi_tile_geometry(int q, int N, int nwhole, int ninner, int sms, PiTileGeo* 
   return found;
 }
 
-static cudaError_t sm_count(int* sms) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
-}
-
 template <bool DISS, int MODE>
-static cudaError_t launch_pi_tma_t(cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st, int b0,
-                                   int nb) {
+static cudaError_t launch_pi_tma_t(cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st, const PiLaunch& L) {
   using namespace pitma;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(rhs_pi_tma_kernel<DISS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM);
+  if (L.first) {
+    const cudaError_t e = cudaFuncSetAttribute(rhs_pi_tma_kernel<DISS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               SMEM);
     if (e != cudaSuccess) return e;
-    attr = true;
   }
-  int sms = 0;
-  cudaError_t e = sm_count(&sms);
-  if (e != cudaSuccess) return e;
-  const int tiles = MODE == MODE_STAGE ? a.nptiles : nb * TILES;
-  rhs_pi_tma_kernel<DISS, MODE><<<(unsigned)(tiles < sms ? tiles : sms), THREADS, SMEM, s>>>(a, M, st, b0, tiles);
+  const int tiles = MODE == MODE_STAGE ? a.nptiles : L.nb * TILES;
+  rhs_pi_tma_kernel<DISS, MODE><<<(unsigned)std::min(tiles, L.sms), THREADS, SMEM, s>>>(a, M, st, L.b0, tiles);
   return cudaGetLastError();
 }
 
-// The Pi kernel over the whole blocks b0 .. b0 + nb - 1 (q = 4, N = 32, FP64).
+// The Pi kernel over the whole blocks of the launch (q = 4, N = 32, FP64).
 cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
-                          int b0, int nb) {
-  if (diss) return mode == MODE_DU ? launch_pi_tma_t<true, MODE_DU>(s, a, M, st, b0, nb)
-                                   : launch_pi_tma_t<true, MODE_STAGE>(s, a, M, st, b0, nb);
-  return mode == MODE_DU ? launch_pi_tma_t<false, MODE_DU>(s, a, M, st, b0, nb)
-                         : launch_pi_tma_t<false, MODE_STAGE>(s, a, M, st, b0, nb);
+                          const PiLaunch& L) {
+  if (diss) return mode == MODE_DU ? launch_pi_tma_t<true, MODE_DU>(s, a, M, st, L)
+                                   : launch_pi_tma_t<true, MODE_STAGE>(s, a, M, st, L);
+  return mode == MODE_DU ? launch_pi_tma_t<false, MODE_DU>(s, a, M, st, L)
+                         : launch_pi_tma_t<false, MODE_STAGE>(s, a, M, st, L);
 }
 
-// The tile Pi kernel over the whole blocks b0 .. b0 + nb - 1 (FP64).
+// The tile Pi kernel over the whole blocks of the launch (FP64).
 cudaError_t launch_pi_tile(int q, bool diss, int mode, cudaStream_t s, const RhsArgs& a, const TmaMaps& M, WaitStatus st,
-                           const PiTileGeo& g, int b0, int nb) {
-  int sms = 0;
-  const cudaError_t e = sm_count(&sms);
-  if (e != cudaSuccess) return e;
-  const int tiles = mode == MODE_STAGE ? a.nptiles : nb * g.tiles_y * g.tiles_z;
-  const unsigned grid = (unsigned)std::min(tiles, sms);
+                           const PiTileGeo& g, const PiLaunch& L) {
+  const int tiles = mode == MODE_STAGE ? a.nptiles : L.nb * g.tiles_y * g.tiles_z;
+  const unsigned grid = (unsigned)std::min(tiles, L.sms);
   switch (q) {
-    case 2: return launch_pi_tile_q2(diss, mode, grid, s, a, M, st, g, b0, tiles);
-    case 4: return launch_pi_tile_q4(diss, mode, grid, s, a, M, st, g, b0, tiles);
-    case 6: return launch_pi_tile_q6(diss, mode, grid, s, a, M, st, g, b0, tiles);
-    default: return launch_pi_tile_q8(diss, mode, grid, s, a, M, st, g, b0, tiles);
+    case 2: return launch_pi_tile_q2(diss, mode, grid, s, a, M, st, g, L, tiles);
+    case 4: return launch_pi_tile_q4(diss, mode, grid, s, a, M, st, g, L, tiles);
+    case 6: return launch_pi_tile_q6(diss, mode, grid, s, a, M, st, g, L, tiles);
+    default: return launch_pi_tile_q8(diss, mode, grid, s, a, M, st, g, L, tiles);
   }
 }
 

@@ -18,6 +18,14 @@ struct WaitStatus {
   long long limit;  // polls a wait may make (negative: give up at once, which tests use)
 };
 
+// a launch of one of the staged Pi kernels over the blocks [b0, b0 + nb) on a device of `sms` SMs; first: the problem's
+// first launch of its form, which tells the device how much shared memory the kernel may ask for (the attribute is the
+// device's, and a problem stays on one)
+struct PiLaunch {
+  int b0, nb, sms;
+  bool first;
+};
+
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
