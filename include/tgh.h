@@ -232,10 +232,11 @@ int tgh_step_batched(tgh_problem* p, double* u, double t, double dt, int nsteps)
  *   threads     CTA size of the head and one-point Pi kernels, 64 or 128;
  *   pi_mb       the one-point Pi kernel's resident CTAs per SM (its launch bound), 3, 4 or 5.
  * All variants give the same bits. A change drops the batched form's captured graph.
- * tgh_set_wait_limit bounds the polls of every device-side wait (the TMA kernel's waits for its
- * copies); a wait that runs out records TGH_ERR_TIMEOUT and its CTA writes nothing. A negative
- * limit gives up at once (for tests). tgh_device_status synchronizes the problem's stream and
- * returns (and clears) TGH_ERR_TIMEOUT if a wait gave up since the last call. */
+ * tgh_set_wait_limit bounds the polls of every device-side wait (the staged Pi kernels' waits for
+ * their copies); a wait that runs out records TGH_ERR_TIMEOUT and its CTA writes nothing. A negative
+ * limit gives up at once (for tests). From then on every verb that goes on from the state, and the one
+ * that waits for the kernel, returns TGH_ERR_TIMEOUT. tgh_device_status synchronizes the problem's
+ * stream and returns (and clears) TGH_ERR_TIMEOUT if a wait gave up since the last call. */
 enum { TGH_PI_L1 = 0, TGH_PI_TMA = 1, TGH_PI_TILE = 2 };
 int tgh_set_variant(tgh_problem* p, int pi_variant, int threads, int pi_mb);
 int tgh_get_variant(const tgh_problem* p, int* pi_variant, int* threads, int* pi_mb);

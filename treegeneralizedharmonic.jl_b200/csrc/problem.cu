@@ -162,7 +162,10 @@ struct tgh_problem {
   int threads = 128;  // CTA size of the head and one-point Pi kernels
   int pi_mb = 4;      // the one-point Pi kernel's resident CTAs per SM (its launch bound)
   std::vector<std::pair<const double*, TmaMaps>> tma_maps;
-  int* dev_err = nullptr;                 // a bounded device wait that gave up records it here
+  // a bounded device wait that gave up records it here: pinned host memory, and its device address, so that every
+  // verb can look at it without waiting for the GPU
+  volatile int* wait_word = nullptr;
+  int* dev_err = nullptr;
   // the blocks interior_kernel visits: those that can hold a point with r < r_1 at some time of
   // [lo, hi]; one list for direct launches, one for the captured graph (built before capture)
   struct BlockList {
@@ -191,6 +194,20 @@ struct tgh_problem {
 static int fail(tgh_problem* p, int code, const std::string& msg) {
   p->err = msg;
   return code;
+}
+
+// whether a bounded device wait has given up since the last tgh_device_status: the state on the device is then
+// unfinished, and every verb that goes on from it refuses
+static int waits_ok(tgh_problem* p) {
+  const int code = p->wait_word ? *p->wait_word : 0;
+  return code == 0 ? TGH_OK
+                   : fail(p, code, "a bounded wait inside a kernel gave up (its results were not written); "
+                                   "tgh_device_status clears this");
+}
+// the stream's work done, none of its waits given up
+static int finished(tgh_problem* p) {
+  CK(cudaStreamSynchronize(p->stream));
+  return waits_ok(p);
 }
 
 // doubles in one of the problem's working arrays (rows padded to the pitch Wx), and in the
@@ -784,6 +801,7 @@ static int launch_hooks(tgh_problem* p, double* work, double t) {
 
 // ---- the fill: stage 0 (copies, hooks), then prolongation level by level ----
 static int launch_fill(tgh_problem* p, const double* src, bool from_work, double* work, double t) {
+  if (int st = waits_ok(p)) return st;
   const int T = 256;
   if (!from_work && p->nranks > 1)
     return fail(p, TGH_ERR_ARG, "a sharded problem is filled through its exchange phases (tgh_shard_*), not from u");
@@ -931,6 +949,7 @@ static int launch_interior(tgh_problem* p, const RhsArgs& a, int mode, cudaStrea
 }
 
 static int launch_rhs(tgh_problem* p, const RhsArgs& a, int mode) {
+  if (int st = waits_ok(p)) return st;
   if (p->intr && !p->interior_done) {
     int s = launch_interior(p, a, mode, p->stream);
     if (s) return s;
@@ -1027,7 +1046,7 @@ static int apply_bounds_impl(tgh_problem* p, double* u, double t, const tgh_boun
   CK(launch_bounds_projection(p->stream, p->cs, a));
   unsigned long long h[3];
   CK(cudaMemcpyAsync(h, p->bcounts, sizeof(h), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   *fired = (long)h[0];
   *nonfinite = (long)h[1];
   double r;
@@ -1199,8 +1218,11 @@ static int setup_device(tgh_problem* p) {
   CK(alloc_work(p, &p->work));
   CK(cudaMalloc(&p->scratch, 2 * sizeof(unsigned long long)));
   CK(cudaMalloc(&p->bcounts, 3 * sizeof(unsigned long long)));
-  CK(cudaMalloc(&p->dev_err, sizeof(int)));
-  CK(cudaMemsetAsync(p->dev_err, 0, sizeof(int), p->stream));
+  void* word = nullptr;
+  CK(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+  p->wait_word = (volatile int*)word;
+  *p->wait_word = 0;
+  CK(cudaHostGetDevicePointer((void**)&p->dev_err, word, 0));
   CK(cudaMalloc(&p->coef, (size_t)NCOEF * p->SX * p->nb * sizeof(double)));
   p->npart = (int)grid_for(p->npts, 128);
   CK(cudaMalloc(&p->part, (3 * (size_t)p->npart + 2) * sizeof(double)));
@@ -1254,7 +1276,7 @@ void tgh_problem_destroy(tgh_problem* p) {
   for (double* w : {p->work, p->W1, p->W2, p->twork})
     if (w) cudaFree(w - p->XO);
   void* bufs[] = {p->beyond, p->pruns, p->ptiles, p->Hsrc, p->tw, p->tf, p->blk, p->primary, p->runs, p->gpts, p->hooks, p->hook_cache, p->scratch,
-                  p->bcounts, p->dev_err, p->ilist.dev, p->ilist_graph.dev,
+                  p->bcounts, p->ilist.dev, p->ilist_graph.dev,
                   p->part, p->coef, p->diag, p->dpart, p->ind, p->ind_tol, p->ind_counts, p->ind_boxes,
                   p->k, p->acc, p->y, p->u0, p->bacc, p->kt, p->acct, p->yt,
                   p->adj_cot, p->adj_mu, p->adj_part, p->adj_y[0], p->adj_y[1], p->adj_y[2], p->adj_a,
@@ -1267,6 +1289,8 @@ void tgh_problem_destroy(tgh_problem* p) {
     if (pp) cudaFree(pp);
   for (auto* pp : p->ptpts)
     if (pp) cudaFree(pp);
+  // after the cudaFrees, which wait for the device: no kernel can still write the word
+  if (p->wait_word) cudaFreeHost((void*)p->wait_word);
   delete p;
 }
 
@@ -1300,7 +1324,7 @@ int tgh_copy_work_blocks(tgh_problem* p, int b0, int nblocks, double* dst) {
   CK(cudaMemcpy2DAsync(dst, (size_t)p->Wd * sizeof(double), p->work + (size_t)p->Wv * NV * b0,
                        (size_t)p->Wx * sizeof(double), (size_t)p->Wd * sizeof(double), rows, cudaMemcpyDeviceToDevice,
                        p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   return TGH_OK;
 }
 
@@ -1382,7 +1406,7 @@ int tgh_constraint_norms(tgh_problem* p, int weighting, int at_level, double* ou
   CK(cudaGetLastError());
   double r[17];
   CK(cudaMemcpyAsync(r, fold, sizeof(r), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   const double vol = r[0];
   double l2[8];
   for (int s = 0; s < 8; ++s) l2[s] = vol == 0.0 ? 0.0 : std::sqrt(r[1 + s] / vol);
@@ -1411,7 +1435,7 @@ int tgh_tau(tgh_problem* p, const double* u, double t, int mask, double eps, dou
   CK(cudaGetLastError());
   unsigned long long bits[11];
   CK(cudaMemcpyAsync(bits, p->ind, 10 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   double sc = 0.0;
   for (int v = 0; v < NC; ++v) {
     double x;
@@ -1424,7 +1448,7 @@ int tgh_tau(tgh_problem* p, const double* u, double t, int mask, double eps, dou
   tau_kernel<<<nb, 128, 0, p->stream>>>(a, p->cs, floor4, p->ind + 10);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(&bits[10], p->ind + 10, sizeof(unsigned long long), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   out[10] = sc;
   std::memcpy(&out[11], &bits[10], sizeof(double));
   return TGH_OK;
@@ -1448,7 +1472,7 @@ int tgh_firing(tgh_problem* p, int ntol, const double* tol, int* counts, int* bo
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(counts, p->ind_counts, n * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
   CK(cudaMemcpyAsync(boxes, p->ind_boxes, 6 * (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   return TGH_OK;
 }
 
@@ -1467,7 +1491,7 @@ int tgh_transfer(tgh_problem* dst, tgh_problem* src, const double* u_src, double
     same = same && dst->lo[d] == src->lo[d] && dst->cells0[d] == src->cells0[d] && dst->periodic[d] == src->periodic[d];
   if (!same) return fail(dst, TGH_ERR_ARG, "the two problems differ in order, block size or root grid");
   int s = prepare_impl(src, u_src, t, "tgh_transfer (as its source)");
-  if (s) return s;
+  if (s) return fail(dst, s, src->err);
   const int G = src->G, Wd = src->Wd, Wx = src->Wx, P = src->q + 2;
   std::vector<CopyPt> cp;
   std::vector<ProlongPt> pp;
@@ -1561,6 +1585,7 @@ int tgh_transfer(tgh_problem* dst, tgh_problem* src, const double* u_src, double
     CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(src->stream));
+  if ((s = waits_ok(src))) return fail(dst, s, src->err);
   return TGH_OK;
 }
 
@@ -1610,13 +1635,10 @@ int tgh_set_wait_limit(tgh_problem* p, long long polls) {
 }
 
 int tgh_device_status(tgh_problem* p) {
-  int h = 0;
-  CK(cudaMemcpyAsync(&h, p->dev_err, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
   CK(cudaStreamSynchronize(p->stream));
-  if (h == 0) return TGH_OK;
-  CK(cudaMemsetAsync(p->dev_err, 0, sizeof(int), p->stream));
-  CK(cudaStreamSynchronize(p->stream));
-  return fail(p, h, "a bounded wait inside a kernel gave up (its results were not written)");
+  const int s = waits_ok(p);
+  *p->wait_word = 0;
+  return s;
 }
 
 int tgh_rhs(tgh_problem* p, double* du, double t, const double* matter) {
@@ -1756,7 +1778,7 @@ int tgh_max_speed(tgh_problem* p, const double* u, double t, double* lambda) {
   CK(cudaGetLastError());
   unsigned long long h[2];
   CK(cudaMemcpyAsync(h, p->scratch, sizeof(h), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   if (h[1] > 0)
     return fail(p, TGH_ERR_NONFINITE, "the state at t = " + std::to_string(t) + " is not finite where it is evolved: " +
                                           std::to_string(h[1]) + " values at evolved points are NaN or Inf");
@@ -1778,7 +1800,7 @@ int tgh_error_norm(tgh_problem* p, const double* u, double t, double* l2, double
   CK(cudaGetLastError());
   double h[2];
   CK(cudaMemcpyAsync(h, p->part + 3 * (size_t)p->npart, sizeof(h), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   *l2 = h[0];
   *linf = h[1];
   return TGH_OK;
@@ -2193,6 +2215,7 @@ int tgh_shard_rhs(tgh_problem* p, int stage, double t, double dt) {
 }
 
 int tgh_shard_end(tgh_problem* p, double* u) {
+  if (int st = waits_ok(p)) return st;
   if (!p->W1) return fail(p, TGH_ERR_ARG, "tgh_shard_begin has not been called");
   gather_kernel<<<grid_for(p->npts, 256), 256, 0, p->stream>>>(p->work, u, p->geo, p->npts, p->beyond);
   CK(cudaGetLastError());
@@ -2233,6 +2256,7 @@ int tgh_time_rhs(tgh_problem* p, const double* u, double t, int mode, int nlaunc
   CK(cudaEventElapsedTime(&ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if ((s = waits_ok(p))) return s;
   *ms_per_launch = ms / nlaunch;
   return TGH_OK;
 }
@@ -2351,7 +2375,7 @@ int tgh_tangent_error_norm(tgh_problem* p, const double* u, const double* ut, do
   CK(cudaGetLastError());
   std::vector<double> h(3 * (size_t)p->npart);
   CK(cudaMemcpyAsync(h.data(), p->part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   double a = 0.0, b = 0.0, w = 0.0;  // summed in block order, on the host
   for (int i = 0; i < p->npart; ++i) {
     a += h[3 * i];
@@ -2418,7 +2442,7 @@ static int vjp_rhs(tgh_problem* p, const double* y, double t, const double* a, d
   if (th3) {
     std::vector<double> h(3 * (size_t)p->npart);
     CK(cudaMemcpyAsync(h.data(), p->adj_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-    CK(cudaStreamSynchronize(p->stream));
+    if (int st = finished(p)) return st;
     for (int i = 0; i < p->npart; ++i)  // in block order, on the host
       for (int k = 0; k < 3; ++k) th3[k] += h[3 * i + k];
   }
@@ -2476,7 +2500,7 @@ int tgh_adjoint_error_norm(tgh_problem* p, const double* u, double t, double* l2
   CK(cudaGetLastError());
   std::vector<double> h(3 * (size_t)p->npart);
   CK(cudaMemcpyAsync(h.data(), p->part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-  CK(cudaStreamSynchronize(p->stream));
+  if (int st = finished(p)) return st;
   double a = 0.0, w = 0.0;
   for (int i = 0; i < p->npart; ++i) {
     a += h[3 * i];

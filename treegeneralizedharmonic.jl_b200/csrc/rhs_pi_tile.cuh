@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
   if (!ok) {
     // a wait gave up: record it, let the copies already issued land, bounded, then leave without writing further
     if (tid == 0) {
-      atomicExch(stat.err, TGH_ERR_TIMEOUT);
+      stat.gave_up();
       auto issued = [&](int c) { return blockIdx.x + (long)(c / NC) * gridDim.x < ntiles; };
       for (int c = n; c < pend_h; ++c)
         if (issued(c)) mbar_wait(bar + 8 * stage_of(c), phase_of(c), 1ll << 24);

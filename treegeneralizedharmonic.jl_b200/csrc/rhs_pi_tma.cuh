@@ -27,7 +27,8 @@
 //
 // Waits on the mbarriers are bounded: a wait that gives up records TGH_ERR_TIMEOUT in the
 // launch's status word, waits (bounded again) for the copies it issued to land, and the CTA
-// returns without writing further; the host reads the word after the step.
+// returns without writing further; the next verb on the problem, or the one that waits for this launch, reads the
+// word and refuses.
 #pragma once
 #include "rhs.cuh"
 #include "tma.cuh"
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(pitma::THREADS)
   if (!ok) {
     // a wait gave up: record it, let the copies already issued (copy n, and copy 1 when n = 0)
     // land, bounded, then leave without writing further
-    if (tid == 0) atomicExch(stat.err, TGH_ERR_TIMEOUT);
+    if (tid == 0) stat.gave_up();
     const long long drain = 1ll << 24;
     mbar_wait(cta.bar + 8 * (cta.n & 1), (cta.n >> 1) & 1, drain);
     if (cta.n == 0) mbar_wait(cta.bar + 8, 0, drain);

@@ -14,8 +14,12 @@ struct TmaMaps {
 };
 
 struct WaitStatus {
-  int* err;         // TGH_ERR_TIMEOUT is stored here by a wait that gives up
+  int* err;         // in the host's memory: TGH_ERR_TIMEOUT is stored here by a wait that gives up
   long long limit;  // polls a wait may make (negative: give up at once, which tests use)
+  __device__ __forceinline__ void gave_up() const {
+    *(volatile int*)err = TGH_ERR_TIMEOUT;
+    __threadfence_system();
+  }
 };
 
 // a launch of one of the staged Pi kernels over the blocks [b0, b0 + nb) on a device of `sms` SMs; first: the problem's
