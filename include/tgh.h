@@ -234,7 +234,7 @@ int tgh_step_batched(tgh_problem* p, double* u, double t, double dt, int nsteps)
  * All variants give the same bits. A change drops the batched form's captured graph.
  * tgh_set_wait_limit bounds the polls of every device-side wait (the staged Pi kernels' waits for
  * their copies); a wait that runs out records TGH_ERR_TIMEOUT and its CTA writes nothing. A negative
- * limit gives up at once (for tests). From then on every verb that goes on from the state, and the one
+ * limit gives up at once (for tests; -2 in the tile kernel only at the second of a component's two boxes). From then on every verb that goes on from the state, and the one
  * that waits for the kernel, returns TGH_ERR_TIMEOUT. tgh_device_status synchronizes the problem's
  * stream and returns (and clears) TGH_ERR_TIMEOUT if a wait gave up since the last call. */
 enum { TGH_PI_L1 = 0, TGH_PI_TMA = 1, TGH_PI_TILE = 2 };

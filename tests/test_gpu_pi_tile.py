@@ -2,6 +2,8 @@
 second point of a pair past a block's end (odd and even edges, 9 to 96), the smallest and largest halos (q = 2 and
 8), one staging buffer and two, blocks that keep all, some or none of their upper faces, a layer and a frozen core,
 no dissipation. The meshes hold enough points for the kernel to be the one that runs."""
+import time
+
 import pytest
 import torch
 
@@ -63,20 +65,25 @@ def test_tile_variant_is_refused_where_it_does_not_apply(tgh):
         P.close()
 
 
+@pytest.mark.parametrize("limit", [-1, -2])
 @pytest.mark.parametrize("q,N", [(4, 16), (8, 27)])
-def test_a_tile_wait_that_runs_out_is_reported(tgh, q, N):
-    """With two staging buffers (q = 4) and with one (q = 8): every CTA gives up on its first copy, lets the
-    copies it issued land and leaves."""
+def test_a_tile_wait_that_runs_out_is_reported(tgh, q, N, limit):
+    """With two staging buffers (q = 4) and with one (q = 8): every CTA gives up on the first of its first two copies,
+    or (limit -2) on the second, when h's box may have been refilled already; it lets the copies that it issued land
+    and leaves at once: a wait for a copy never issued would go on for 2^24 polls."""
     case = tgh.gauge_wave_case(eps_ko=0.5, gamma0=1.0)
     P = tgh.GHProblem(case, tgh.gh_forest(case, N, 3), q, margin_check=False, tuned=False)
     u = P.initial_state(P.statevector(), 0.25)
     ref, du = torch.zeros_like(u), torch.zeros_like(u)
     P.gh_rhs(ref, u, 0.25)
-    P.set_wait_limit(-1)
+    torch.cuda.synchronize()
+    P.set_wait_limit(limit)
+    start = time.perf_counter()
     P.gh_rhs(du, u, 0.25)
     with pytest.raises(tgh._abi.TGHError) as e:
         P.device_status()
     assert e.value.code == tgh._abi.TGH_ERR_TIMEOUT
+    assert time.perf_counter() - start < 0.1  # the launches take under a millisecond
     P.set_wait_limit(1 << 26)
     P.gh_rhs(du, u, 0.25)
     P.device_status()

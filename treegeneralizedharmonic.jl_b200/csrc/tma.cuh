@@ -15,7 +15,8 @@ struct TmaMaps {
 
 struct WaitStatus {
   int* err;         // in the host's memory: TGH_ERR_TIMEOUT is stored here by a wait that gives up
-  long long limit;  // polls a wait may make (negative: give up at once, which tests use)
+  long long limit;  // polls a wait may make; for tests, negative: give up at once, -2: at a component's second box only
+  __device__ __forceinline__ long long first_limit() const { return limit == -2 ? 1ll << 26 : limit; }
   __device__ __forceinline__ void gave_up() const {
     *(volatile int*)err = TGH_ERR_TIMEOUT;
     __threadfence_system();
