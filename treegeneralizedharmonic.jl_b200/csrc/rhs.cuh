@@ -619,31 +619,32 @@ __device__ __forceinline__ void interior_point(const Case& cs, const RhsArgs& A,
 // where the head and Pi kernels will add the stencil part. Kept out of the head kernel so that
 // its registers serve the main path alone.
 //
-// A CTA looks at INTERIOR_CHUNK consecutive points of a block, lists the frozen ones from the front and the
-// layer's from the back of a shared array, and then works through the list: a sphere fills few warps of
-// consecutive points whole (13.7 of 32 lanes, a thread per point), and a frozen point's work and a
-// layer point's are different code. A stage of the moving hole on 232 blocks: 0.83 ms (1.39 ms, a thread per
-// point); of the :fitted interior on 2472 blocks of 8^3: 0.27 ms (0.76 ms, its loads one variable at a time).
-constexpr int INTERIOR_CHUNK = 512;
+// A CTA looks at `chunk` consecutive points of a block, lists the frozen ones from the front and the layer's from the
+// back of a shared array, and then works through the array: a sphere fills few warps of consecutive points whole (13.7
+// of 32 lanes, a thread per point), and a frozen point's work and a layer point's are different code. A stage of the
+// moving hole on 232 blocks: 0.83 ms (1.39 ms, a thread per point); of the :fitted interior on 2472 blocks of 8^3:
+// 0.27 ms (0.76 ms, its loads one variable at a time). Few CTAs get few points each (launch_interior), as a thread works
+// through its share one point after the other.
+constexpr int INTERIOR_CHUNK = 512;  // the most
 template <int MODE>
-__global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsArgs A, const int* __restrict__ blocks) {
+__global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsArgs A, const int* __restrict__ blocks, int chunk) {
   __shared__ short list[INTERIOR_CHUNK];
   __shared__ int count[2];  // frozen, layer
   const int S = A.N1 * A.N1 * A.N1;
-  const int per = (S + INTERIOR_CHUNK - 1) / INTERIOR_CHUNK;
-  const int b = blocks[blockIdx.x / per], base = (blockIdx.x % per) * INTERIOR_CHUNK;
+  const int per = (S + chunk - 1) / chunk;
+  const int b = blocks[blockIdx.x / per], base = (blockIdx.x % per) * chunk;
   if ((long)b * S < A.p0 || (long)b * S >= A.p1) return;  // launches cover whole blocks
   if (threadIdx.x < 2) count[threadIdx.x] = 0;
   __syncthreads();
   const double rf = cs.interior == TGH_INT_PASTED ? cs.r1 : cs.r0;
   auto at = [&](int ip) { return point_at(A, b, ip % A.N1, (ip / A.N1) % A.N1, ip / (A.N1 * A.N1)); };
-  for (int e = threadIdx.x; e < INTERIOR_CHUNK && base + e < S; e += 128) {
+  for (int e = threadIdx.x; e < chunk && base + e < S; e += 128) {
     const double r = interior_radius(cs, A.t, at(base + e).x);
     if (r >= cs.r1) continue;
     if (r < rf)
       list[atomicAdd(&count[0], 1)] = (short)e;
     else
-      list[INTERIOR_CHUNK - 1 - atomicAdd(&count[1], 1)] = (short)e;
+      list[chunk - 1 - atomicAdd(&count[1], 1)] = (short)e;
   }
   __syncthreads();
   const int nf = count[0], nl = count[1];
@@ -651,8 +652,9 @@ __global__ void __launch_bounds__(128) interior_kernel(const Case cs, const RhsA
     const PointIdx q = at(base + list[m]);
     interior_point<MODE>(cs, A, q, interior_radius(cs, A.t, q.x), true);
   }
-  for (int m = threadIdx.x; m < nl; m += 128) {
-    const PointIdx q = at(base + list[INTERIOR_CHUNK - 1 - m]);
+  // from the last thread on: the warps that had no frozen point take the layer's first
+  for (int m = 127 - threadIdx.x; m < nl; m += 128) {
+    const PointIdx q = at(base + list[chunk - 1 - m]);
     interior_point<MODE>(cs, A, q, interior_radius(cs, A.t, q.x), false);
   }
 }
