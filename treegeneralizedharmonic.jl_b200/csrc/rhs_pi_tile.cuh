@@ -158,10 +158,10 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
   __syncthreads();
 
   const long S = (long)N1 * N1 * N1, SX = (long)A.NX * N1 * N1, sv = (long)A.Wx * A.Wd * A.Wd;
-  int n = 0;        // copies consumed
-  int gave_up = 0;  // 1: the wait for copy n of h did, 2: for copy n of Pi
+  int n = 0, pend_h = g.stages, pend_p = g.stages;  // copies consumed; issued of h and of Pi (thread 0's view)
+  bool ok = true;
 #pragma unroll 1
-  for (int t = blockIdx.x; !gave_up && t < ntiles; t += gridDim.x) {
+  for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x) {
     const PiTile T = tile_at(t);
     const int ex = N1 - 1 + (T.full & 1), ey = N1 - 1 + ((T.full >> 1) & 1), ez = N1 - 1 + (T.full >> 2);
     const int TY = g.shape[T.shape].TY, TZ = g.shape[T.shape].TZ, ROWS = TY * TZ;
@@ -222,10 +222,13 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
       // barrier after the component before: its stage and the inner sums may now be refilled.
       bool got = mbar_wait(bar + 8 * st, ph, stat.first_limit());
       if (!__syncthreads_and(got)) {
-        gave_up = 1;
+        ok = false;
         break;
       }
-      if (g.stages == 2 && n >= 1 && tid == 0) issue(n + 1, true, true);
+      if (g.stages == 2 && n >= 1) {
+        if (tid == 0) issue(n + 1, true, true);
+        pend_h = pend_p = n + 2;
+      }
       const double* H = reinterpret_cast<const double*>(smem + st * g.stage);
       const double* P = reinterpret_cast<const double*>(smem + st * g.stage + g.p_off);
       double s[2], p2[2], hd1[3][2], ko[2];
@@ -281,6 +284,7 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
       if (g.stages == 1) {
         __syncthreads();  // h's box is read
         if (tid == 0) issue(n + 1, true, false);
+        pend_h = n + 2;
       }
       got = mbar_wait(bar + 16 + 8 * st, ph, stat.limit);
       if (active && got) {
@@ -335,10 +339,13 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
       }
       // the inner sums are written (and Pi's box is read)
       if (!__syncthreads_and(got)) {
-        gave_up = 2;
+        ok = false;
         break;
       }
-      if (g.stages == 1 && tid == 0) issue(n + 1, false, true);
+      if (g.stages == 1) {
+        if (tid == 0) issue(n + 1, false, true);
+        pend_p = n + 2;
+      }
       if (!any) continue;
       {
         double mxy[2], mxz[2];
@@ -387,18 +394,16 @@ __global__ void __launch_bounds__(PI_TILE_THREADS)
       }
     }
   }
-  if (gave_up) {
-    // record it, let the copies already issued land, bounded, then leave without writing further. Issued are copy n,
-    // with two stages copy 1 from the start, and copy n + 1 (with one stage h's) once copy n of h was consumed. That one
-    // is not waited for again: with one stage copy n + 1 is on its barrier, and once it has landed a wait for copy n's
-    // phase would wait for a copy that is never issued.
+  if (!ok) {
+    // a wait gave up: record it, let the copies already issued land, bounded, then leave without writing further. With
+    // one stage, copy n + 1 of h is issued on the barrier of copy n once that is consumed, and when it has landed a wait
+    // for copy n's phase would wait for a copy that is never issued: only copy n + 1 is waited for then.
     if (tid == 0) {
       stat.gave_up();
-      const int end = g.stages == 2 ? max(2, n + gave_up) : n + gave_up, end_pi = g.stages == 2 ? end : n + 1;
       auto issued = [&](int c) { return blockIdx.x + (long)(c / NC) * gridDim.x < ntiles; };
-      for (int c = n + gave_up - 1; c < end; ++c)
+      for (int c = g.stages == 1 ? pend_h - 1 : n; c < pend_h; ++c)
         if (issued(c)) mbar_wait(bar + 8 * stage_of(c), phase_of(c), 1ll << 24);
-      for (int c = n; c < end_pi; ++c)
+      for (int c = n; c < pend_p; ++c)
         if (issued(c)) mbar_wait(bar + 16 + 8 * stage_of(c), phase_of(c), 1ll << 24);
     }
     __syncthreads();  // the shared arrays outlive their copies
