@@ -28,3 +28,40 @@ def test_interior_on_small_meshes(tgh, oracle, N, variant, v):
     case = tgh.kerr_schild_case(a=0.7, v=v, halfwidth=2.0, variant=variant, gauge="algebraic")
     # the bound of the right-hand side's parity everywhere
     assert _rhs_error(tgh, oracle, case, tgh.gh_forest(case, N, 2), 4, 0.3) < 1e-12
+
+
+# the one-point Pi kernel's registers: a block's launch is below the line (27 CTAs), the mesh's of 1,688 above it
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("q", [2, 4, 6, 8])
+@pytest.mark.parametrize("eps", [0.5, 0.0])
+def test_register_bounds_give_the_same_bits(tgh, q, precision, eps):
+    case = tgh.gauge_wave_case(eps_ko=eps, gamma0=1.0)
+    P = tgh.GHProblem(case, tgh.gh_forest(case, 14, 4), q, margin_check=False, precision=precision, tuned=False)
+    if precision == "fp64":
+        P.set_variant(pi="l1")
+    u = P.initial_state(P.statevector(), 0.0)
+    u += 1e-6 * torch.randn(u.shape, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    P.settle(u, 0.0)
+    a, b = u.clone(), u.clone()
+    P.rk4_step(a, 0.0, 1e-3)
+    P.rk4_step_blocks(b, 0.0, 1e-3)
+    assert torch.isfinite(a).all() and torch.equal(a, b)
+    P.close()
+
+
+# the batched form below the line (138 CTAs of runs) against the oracle
+@pytest.mark.parametrize("q", [2, 4, 6, 8])
+def test_batched_step_on_a_small_mesh(tgh, oracle, q):
+    case = tgh.gauge_wave_case(eps_ko=0.5, gamma0=1.0)
+    f = tgh.gh_forest(case, 12, 2)
+    P = tgh.GHProblem(case, f, q, margin_check=False, tuned=False)
+    O = oracle.problem(case, f, q)
+    u = O.initial_state(O.statevector(), 0.0) + tgh.perturbation(f, amplitude=1e-6, seed=11)
+    a = torch.from_numpy(u).cuda()
+    P.settle(a, 0.0)  # the copies of a shared point agree: the batched form starts from the primaries
+    u = a.cpu().numpy()
+    dt = 0.25 * f.h0 / 4
+    P.step_batched(a, 0.0, dt, 1)
+    O.rk4_step(u, 0.0, dt)
+    assert np.abs(a.cpu().numpy() - u).max() < 1e-12  # the parity bound of a step on states of order one
+    P.close()

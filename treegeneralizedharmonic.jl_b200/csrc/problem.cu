@@ -855,11 +855,11 @@ static bool tma_applies(const tgh_problem* p, const RhsArgs& a) {
 }
 
 // Whether a launch takes the tile Pi kernel: the variant chosen, whole blocks, and enough points to fill the GPU with
-// tiles. Where the line lies (us a right-hand side, one-point against tile): at q >= 4 in the plain form 8 blocks of
-// 12^3 (17,576 points) 37 against 54 and of 16^3 (39,304) 52 against 44; in the batched form, whose epilogue both
-// wait for, 8 of 16^3 46 against 47 (q = 4) and 42 against 46 (q = 6), 64 of 16^3 (262,144 computed) 269 against 208
-// and 267 against 253; the batched form's rows of 8 points share banks, 2472 blocks of 8^3 1,582 against 1,584. At
-// q = 2 there is less to share: 8 blocks of 32^3 121 against 131, 27 of 27^3 333 against 269.
+// tiles. Where the line lies (us a right-hand side, one-point against tile): at q = 4 in the plain form 8 blocks of
+// 12^3 (17,576 points) 26 against 31 and of 16^3 (39,304) 51 against 41; in the batched form, whose epilogue both
+// wait for, 8 of 16^3 29 against 39 and 27 of 16^3 (110,592 computed) 134 against 106, at q = 6 37 against 43 and 149
+// against 121; the batched form's rows of 8 points share banks, 2472 blocks of 8^3 1,582 against 1,584. At q = 2 there
+// is less to share: 27 of 16^3 74 against 78, 8 of 32^3 121 against 131, 27 of 27^3 333 against 269.
 static bool tile_applies(const tgh_problem* p, const RhsArgs& a, int mode) {
   if (p->pi_variant != PI_TILE || a.p0 % p->S != 0 || a.p1 % p->S != 0) return false;
   const long points = mode == MODE_STAGE ? 128L * a.npruns : a.p1 - a.p0;
@@ -1002,6 +1002,7 @@ static RhsArgs base_args(tgh_problem* p, const double* work, double t) {
   a.nptiles = p->nptiles;
   a.threads = p->threads;
   a.pi_mb = p->pi_mb;
+  a.sms = p->sms;
   return a;
 }
 

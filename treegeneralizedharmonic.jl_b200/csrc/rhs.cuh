@@ -236,7 +236,8 @@ struct RhsArgs {
   const PiTile* ptiles;
   int npruns, nptiles;
   int threads;            // CTA size of the launch (64 or 128)
-  int pi_mb;              // the one-point Pi kernel's resident CTAs per SM (3, 4 or 5)
+  int pi_mb;              // the one-point Pi kernel's resident CTAs per SM (3, 4 or 5; N = 32)
+  int sms;                // of the device
 };
 
 // Where a finished component goes: straight to du (plain form) or into the RK4 stage

@@ -34,6 +34,16 @@ cudaError_t launch_rhs_n(int part, bool intr, cudaStream_t s, const Case& cs, co
       if (a.pi_mb == 3) rhs_pi_kernel<Q, DISS, MODE, T, N1S, 3><<<nb, TH, 0, s>>>(cs, a);
       else if (a.pi_mb == 5) rhs_pi_kernel<Q, DISS, MODE, T, N1S, 5><<<nb, TH, 0, s>>>(cs, a);
       else rhs_pi_kernel<Q, DISS, MODE, T, N1S><<<nb, TH, 0, s>>>(cs, a);
+    } else if constexpr (N1S == 0) {
+      // A launch whose CTAs of 128 threads are all resident at two an SM has no use for the occupancy that 128 registers
+      // a thread buy, and at 255 nothing spills and no address is formed twice; in the batched form at q = 2 that still
+      // pays at three waves of them. us a call at 128 against 255 registers: gh_rhs on 8 blocks of 12^3 (138 CTAs) at
+      // q = 4, 49 against 33, mixed 61 against 37; two batched steps at q = 2 on 27 blocks of 14^3 (594 CTAs) 732
+      // against 623. Above the line gh_rhs on 8 of 20^3 (579 CTAs), mixed at q = 2, 47 against 53; two batched steps on
+      // 27 of 12^3 (378 CTAs), mixed at q = 6, 827 against 851.
+      const long few = MODE == MODE_STAGE && Q == 2 ? 6 : 2;
+      if ((long)nb * TH <= few * 128 * a.sms) rhs_pi_kernel<Q, DISS, MODE, T, N1S, 2><<<nb, TH, 0, s>>>(cs, a);
+      else rhs_pi_kernel<Q, DISS, MODE, T, N1S><<<nb, TH, 0, s>>>(cs, a);
     } else {
       rhs_pi_kernel<Q, DISS, MODE, T, N1S><<<nb, TH, 0, s>>>(cs, a);
     }
