@@ -240,6 +240,11 @@ int tgh_step_batched(tgh_problem* p, double* u, double t, double dt, int nsteps)
 enum { TGH_PI_L1 = 0, TGH_PI_TMA = 1, TGH_PI_TILE = 2 };
 int tgh_set_variant(tgh_problem* p, int pi_variant, int threads, int pi_mb);
 int tgh_get_variant(const tgh_problem* p, int* pi_variant, int* threads, int* pi_mb);
+/* the Pi kernel that one right-hand side over the problem's mesh launches with pi_variant chosen (form 0:
+ * the plain form, 1: the batched form): TGH_PI_TILE runs the one-point kernel on a small mesh */
+int tgh_pi_kernel(const tgh_problem* p, int pi_variant, int form, int* pi);
+/* the points one right-hand side of the batched form computes: those that same-level leaves share once */
+long long tgh_computed_points(const tgh_problem* p);
 int tgh_set_wait_limit(tgh_problem* p, long long polls);
 int tgh_device_status(tgh_problem* p);
 

@@ -93,6 +93,8 @@ SIGNATURES = {
     "tgh_adjoint_rk4_step": (ctypes.c_int, [_VP, _VP, _D, _D, _VP, ctypes.POINTER(_D)]),
     "tgh_get_variant": (ctypes.c_int, [_VP, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
                                        ctypes.POINTER(ctypes.c_int)]),
+    "tgh_pi_kernel": (ctypes.c_int, [_VP, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
+    "tgh_computed_points": (ctypes.c_longlong, [_VP]),
     "tgh_set_wait_limit": (ctypes.c_int, [_VP, ctypes.c_longlong]),
     "tgh_device_status": (ctypes.c_int, [_VP]),
     "tgh_step_batched": (ctypes.c_int, [_VP, _VP, _D, _D, ctypes.c_int]),

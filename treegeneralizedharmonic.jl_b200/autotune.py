@@ -31,17 +31,30 @@ def config_key(problem):
     return f"q{problem.q}_n{problem.forest.N}_{problem.precision}_{'interior' if c.interior else 'nointerior'}"
 
 
+def _tma(problem):
+    return problem.q == 4 and problem.forest.N == 32 and problem.precision == "fp64"
+
+
+def _runs_tile(problem):
+    """Whether the right-hand side that is timed runs the tile kernel under the "tile" variant. A mesh below the tile
+    kernel's line runs the one-point kernel, whose time says nothing about the tile kernel."""
+    if _tma(problem) or problem.precision != "fp64" or not 8 < problem.forest.N <= 96:
+        return False
+    return not hasattr(problem, "pi_kernel") or problem.pi_kernel("batched", "tile") == "tile"
+
+
 def candidates(problem):
+    """The variants that run different kernels on this problem."""
     out = []
+    # the one-point kernel is compiled for several numbers of resident CTAs at N = 32 in FP64 only
+    bounds = (4, 3, 5) if problem.forest.N == 32 and problem.precision == "fp64" else (4,)
+    staged = "tma" if _tma(problem) else "tile" if _runs_tile(problem) else None
     for threads in (128, 64):
-        for mb in (4, 3, 5):
+        for mb in bounds:
             out.append({"pi": "l1", "threads": threads, "pi_mb": mb})
-    if problem.q == 4 and problem.forest.N == 32 and problem.precision == "fp64":
+    if staged:
         for threads in (128, 64):
-            out.append({"pi": "tma", "threads": threads, "pi_mb": 4})
-    elif problem.precision == "fp64" and 8 < problem.forest.N <= 96:
-        for threads in (128, 64):
-            out.append({"pi": "tile", "threads": threads, "pi_mb": 4})
+            out.append({"pi": staged, "threads": threads, "pi_mb": 4})
     return out
 
 
@@ -59,7 +72,7 @@ def tune(problem, u, t=0.0, nlaunch=6, repeats=3, record=True, path=None):
     choice = {k: best[k] for k in ("pi", "threads", "pi_mb")}
     problem.set_variant(**choice)
     res = {"key": config_key(problem), "gpu": gpu_key(), "choice": choice, "sweep": sweep,
-           "points_per_rhs": (problem.forest.N + 1) ** 3 * problem.forest.nblocks}
+           "points_per_rhs": problem.computed_points()}
     if record:
         save_record(res, path)
     return res
@@ -87,9 +100,14 @@ def recorded_choice(problem, path=None):
     rec = json.loads(f.read_text()).get(config_key(problem))
     if not rec:
         return None
-    choice = rec["choice"]
-    tma = problem.q == 4 and problem.forest.N == 32 and problem.precision == "fp64"
-    tile = not tma and problem.precision == "fp64" and problem.forest.N <= 96
-    if (choice["pi"] == "tma" and not tma) or (choice["pi"] == "tile" and not tile):
+    choice = dict(rec["choice"])
+    tile = not _tma(problem) and problem.precision == "fp64" and problem.forest.N <= 96
+    if (choice["pi"] == "tma" and not _tma(problem)) or (choice["pi"] == "tile" and not tile):
         return None
-    return dict(choice)
+    if choice["pi"] == "l1" and hasattr(problem, "pi_kernel") and _runs_tile(problem):
+        # the key holds no size: a one-point choice from a mesh on which the tile kernel was not timed, or from one of
+        # less than half the points (its advantage grows with them), does not stand against the default
+        timed = any(r["pi"] == "tile" for r in rec["sweep"])
+        if not timed or 2 * rec["points_per_rhs"] < problem.computed_points():
+            choice["pi"] = "tile"
+    return choice

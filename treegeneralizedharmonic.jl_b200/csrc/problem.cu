@@ -33,9 +33,9 @@ cudaError_t launch_pi_tma(bool diss, int mode, cudaStream_t s, const RhsArgs& a,
                           const PiLaunch& L);
 }  // namespace tgh
 
-// the Pi kernel a problem launches: the one-point kernel reading through L1, or the pair kernel
-// whose stencil tiles the Tensor Memory Accelerator stages into shared memory (q = 4, N = 32,
-// FP64 only; the one-point kernel serves every other problem)
+// the Pi kernel a problem launches: the one-point kernel reading through L1, or one of the two pair kernels whose
+// stencil tiles the Tensor Memory Accelerator stages into shared memory (FP64): PI_TMA at q = 4, N = 32, PI_TILE at
+// every other order and N <= 96, in launches with enough points for it (pi_kernel_for)
 enum { PI_L1 = TGH_PI_L1, PI_TMA = TGH_PI_TMA, PI_TILE = TGH_PI_TILE };
 
 struct GraphKey {
@@ -129,6 +129,7 @@ struct tgh_problem {
   PointRun* pruns = nullptr;
   PiTile* ptiles = nullptr;
   int npruns = 0, nptiles = 0;
+  long long ncomputed = 0;  // points
   int npart = 0;
   // plain-form RK4 buffers (state layout)
   double *k = nullptr, *acc = nullptr, *y = nullptr, *u0 = nullptr;
@@ -634,6 +635,7 @@ static int build_computed(tgh_problem* p) {
       e[d] = p->N + ((full >> d) & 1);
       n *= e[d];
     }
+    p->ncomputed += n;
     for (int m = 0; m < n; m += 128) runs.push_back(PointRun{b, m << 3 | full});
     if (!tma && !p->tile_geo.threads) continue;
     const bool inner = tma ? !(full & 3) : full == 0;
@@ -849,22 +851,22 @@ static cudaError_t launch_part(tgh_problem* p, int part, int mode, cudaStream_t 
   }
 }
 
-// whether a launch may take the TMA Pi kernel: the variant chosen, its configuration, whole blocks
-static bool tma_applies(const tgh_problem* p, const RhsArgs& a) {
-  return p->pi_variant == PI_TMA && p->q == 4 && p->N == 32 && !p->mixed && a.p0 % p->S == 0 && a.p1 % p->S == 0;
-}
-
-// Whether a launch takes the tile Pi kernel: the variant chosen, whole blocks, and enough points to fill the GPU with
-// tiles. Where the line lies (us a right-hand side, one-point against tile): at q = 4 in the plain form 8 blocks of
+// The Pi kernel of a launch of the given form over `points` points (the computed ones in the batched form), of whole
+// blocks or not, when `variant` is the problem's. The TMA kernel: the variant chosen, its configuration, whole blocks.
+// The tile kernel: the variant chosen, whole blocks, and enough points to fill the GPU with tiles. Where the line lies (us a right-hand side, one-point against tile): at q = 4 in the plain form 8 blocks of
 // 12^3 (17,576 points) 26 against 31 and of 16^3 (39,304) 51 against 41; in the batched form, whose epilogue both
 // wait for, 8 of 16^3 29 against 39 and 27 of 16^3 (110,592 computed) 134 against 106, at q = 6 37 against 43 and 149
 // against 121; the batched form's rows of 8 points share banks, 2472 blocks of 8^3 1,582 against 1,584. At q = 2 there
 // is less to share: 27 of 16^3 74 against 78, 8 of 32^3 121 against 131, 27 of 27^3 333 against 269.
-static bool tile_applies(const tgh_problem* p, const RhsArgs& a, int mode) {
-  if (p->pi_variant != PI_TILE || a.p0 % p->S != 0 || a.p1 % p->S != 0) return false;
-  const long points = mode == MODE_STAGE ? 128L * a.npruns : a.p1 - a.p0;
-  if (p->q == 2) return points >= 500000;
-  return mode == MODE_STAGE ? points >= 100000 && p->N > 8 : points >= 32768;
+static int pi_kernel_for(const tgh_problem* p, int variant, int mode, long points, bool whole) {
+  if (!whole) return PI_L1;
+  if (variant == PI_TMA) return p->q == 4 && p->N == 32 && !p->mixed ? PI_TMA : PI_L1;
+  if (variant != PI_TILE || !p->tile_geo.threads) return PI_L1;
+  if (p->q == 2) return points >= 500000 ? PI_TILE : PI_L1;
+  return (mode == MODE_STAGE ? points >= 100000 && p->N > 8 : points >= 32768) ? PI_TILE : PI_L1;
+}
+static long launch_points(const tgh_problem* p, int mode, long p0, long p1) {
+  return mode == MODE_STAGE ? 128L * p->npruns : p1 - p0;
 }
 
 // the tensor maps of one of the problem's working arrays (made once per array)
@@ -963,14 +965,15 @@ static int launch_rhs(tgh_problem* p, const RhsArgs& a, int mode) {
     if (s) return s;
   }
   CK(launch_part(p, 0, mode, p->stream, a));
-  const bool tma = tma_applies(p, a);
-  if (tma || tile_applies(p, a, mode)) {
+  const int pi = pi_kernel_for(p, p->pi_variant, mode, launch_points(p, mode, a.p0, a.p1),
+                               a.p0 % p->S == 0 && a.p1 % p->S == 0);
+  if (pi != PI_L1) {
     const TmaMaps* M = work_tma_maps(p, a.work);
     if (!M) return TGH_ERR_CUDA;
     bool& launched = p->pi_launched[mode == MODE_STAGE];
     const PiLaunch L{(int)(a.p0 / p->S), (int)((a.p1 - a.p0) / p->S), p->sms, !launched};
     const WaitStatus st{p->dev_err, p->wait_limit};
-    CK(tma ? launch_pi_tma(p->diss, mode, p->stream, a, *M, st, L)
+    CK(pi == PI_TMA ? launch_pi_tma(p->diss, mode, p->stream, a, *M, st, L)
            : launch_pi_tile(p->q, p->diss, mode, p->stream, a, *M, st, p->tile_geo, L));
     launched = true;
     return TGH_OK;
@@ -1633,6 +1636,15 @@ int tgh_get_variant(const tgh_problem* p, int* pi_variant, int* threads, int* pi
   *pi_mb = p->pi_mb;
   return TGH_OK;
 }
+
+int tgh_pi_kernel(const tgh_problem* p, int pi_variant, int form, int* pi) {
+  if (!p || !pi || pi_variant < TGH_PI_L1 || pi_variant > TGH_PI_TILE || form < 0 || form > 1) return TGH_ERR_ARG;
+  const int mode = form ? MODE_STAGE : MODE_DU;
+  *pi = pi_kernel_for(p, pi_variant, mode, launch_points(p, mode, 0, p->npts), true);
+  return TGH_OK;
+}
+
+long long tgh_computed_points(const tgh_problem* p) { return p->ncomputed; }
 
 int tgh_set_wait_limit(tgh_problem* p, long long polls) {
   p->wait_limit = polls;

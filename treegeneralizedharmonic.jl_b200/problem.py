@@ -101,8 +101,21 @@ class GHProblem:
         name = {k: n for n, k in self.PI_VARIANTS.items()}[v.value]
         return {"pi": name, "threads": t.value, "pi_mb": m.value}
 
+    def pi_kernel(self, form="batched", pi=None):
+        """The Pi kernel one right-hand side of the form ("plain" or "batched") launches on this mesh with the
+        variant `pi` (the one set by default): "tile" runs the one-point kernel where the mesh is small."""
+        v = ctypes.c_int()
+        self._check(self.lib.tgh_pi_kernel(self._h, self.PI_VARIANTS[pi or self.variant()["pi"]],
+                                           {"plain": 0, "batched": 1}[form], ctypes.byref(v)))
+        return {k: n for n, k in self.PI_VARIANTS.items()}[v.value]
+
+    def computed_points(self):
+        """The points one right-hand side of the batched form computes."""
+        return int(self.lib.tgh_computed_points(self._h))
+
     def set_wait_limit(self, polls):
-        """Polls a device-side wait may make before it gives up (negative: at once)."""
+        """Polls a device-side wait may make before it gives up (negative: at once; -2: the tile kernel at the
+        second of a component's two boxes only)."""
         self._check(self.lib.tgh_set_wait_limit(self._h, int(polls)))
 
     def device_status(self):
