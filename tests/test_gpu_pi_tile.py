@@ -1,7 +1,7 @@
 """The tile Pi kernel against the one-point kernel, bit for bit, where its tiles can go wrong: rows, planes and the
 second point of a pair past a block's end (odd and even edges, 9 to 96), the smallest and largest halos (q = 2 and
 8), one staging buffer and two, blocks that keep all, some or none of their upper faces, a layer and a frozen core,
-no dissipation. The meshes hold enough points for the kernel to be the one that runs."""
+no dissipation. The meshes hold enough points for the kernel to be the one that runs, which every case checks."""
 import time
 
 import pytest
@@ -10,13 +10,16 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # q, N, roots; periodic gauge wave
-WAVES = [(2, 31, 3), (2, 32, 3), (4, 9, 5), (4, 10, 4), (4, 16, 2), (4, 27, 2), (4, 33, 2), (6, 13, 4), (6, 24, 2),
-         (8, 12, 4), (8, 21, 2), (8, 96, 1)]
+WAVES = [(2, 31, 3), (2, 32, 3), (4, 9, 6), (4, 10, 5), (4, 16, 3), (4, 27, 2), (4, 33, 2), (6, 13, 4), (6, 24, 2),
+         (8, 12, 4), (8, 21, 3), (8, 96, 1)]
 
 
 def _both(tgh, case, forest, q, steps=True):
     P = tgh.GHProblem(case, forest, q, margin_check=False, tuned=False)
     assert P.variant()["pi"] == "tile"
+    assert P.pi_kernel("plain") == "tile" and P.pi_kernel("plain", "l1") == "l1"
+    if steps:
+        assert P.pi_kernel("batched") == "tile" and P.pi_kernel("batched", "l1") == "l1"
     g = torch.Generator(device="cuda").manual_seed(11)
     u = P.initial_state(P.statevector(), 0.0)
     u += 1e-6 * torch.randn(u.shape, dtype=torch.float64, device="cuda", generator=g)
@@ -41,6 +44,24 @@ def _both(tgh, case, forest, q, steps=True):
 def test_tile_kernel_gives_the_one_point_kernels_bits(tgh, q, N, roots, eps):
     case = tgh.gauge_wave_case(eps_ko=eps, gamma0=1.0)
     _both(tgh, case, tgh.gh_forest(case, N, roots), q)
+
+
+@pytest.mark.parametrize("q", [2, 4, 6])
+def test_tile_kernel_on_blocks_of_8_in_the_plain_form(tgh, q):
+    case = tgh.gauge_wave_case(eps_ko=0.5, gamma0=1.0)
+    _both(tgh, case, tgh.gh_forest(case, 8, 9 if q == 2 else 4), q, steps=False)
+
+
+def test_the_rules_line(tgh):
+    """Which kernel a mesh runs on either side of the line, in both forms, and at N = 32, q = 4."""
+    case = tgh.gauge_wave_case(eps_ko=0.5, gamma0=1.0)
+    for q, N, roots, plain, batched in ((4, 12, 2, "l1", "l1"), (4, 16, 2, "tile", "l1"), (4, 16, 3, "tile", "tile"),
+                                        (4, 8, 5, "tile", "l1"), (2, 16, 4, "l1", "l1"), (2, 32, 3, "tile", "tile"),
+                                        (4, 32, 1, "tma", "tma")):
+        P = tgh.GHProblem(case, tgh.gh_forest(case, N, roots), q, margin_check=False, tuned=False)
+        assert (P.pi_kernel("plain"), P.pi_kernel("batched")) == (plain, batched), (q, N, roots)
+        assert P.computed_points() == ((N + 1) ** 3 if roots == 1 else (N * roots) ** 3)
+        P.close()
 
 
 @pytest.mark.parametrize("variant", ["damped", "frozen", "pasted"])
