@@ -133,7 +133,7 @@ static __global__ void __launch_bounds__(128) adjoint_point_kernel(const Case cs
       }
       const Tan gd = damping_rate_t(cs, A.t, q.x, TAN_DAMP_NEAR);
       PhiCotangents g;
-      adjoint_phi_reverse(cs, PhiInputs{hv, d1, dth, Pv, koh, eh, ih, ih2, lh, lP, P1, P2, P0, PKO, W, rho, gd.v, Hl, dHs},
+      adjoint_phi_reverse(cs, PhiInputs{hv, d1, dth, Pv, eh, ih, ih2, lh, lP, P1, P2, P0, PKO, W, rho, gd.v, Hl, dHs},
                           g);
       for (int v = 0; v < NC; ++v) {
         cot(v, AF_HC) = g.h[v];

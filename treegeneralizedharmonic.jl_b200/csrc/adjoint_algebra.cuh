@@ -18,7 +18,7 @@ namespace tgh {
 TGH_HD constexpr double pmul(int n) { return prow(n) == pcol(n) ? 1.0 : 2.0; }
 
 struct PhiInputs {
-  const double *h, *d1, *dth, *Pi, *koh;  // h, d_i h (3 x 10), d_t h, Pi, the dissipation sums of h
+  const double *h, *d1, *dth, *Pi;        // h, d_i h (3 x 10), d_t h, Pi
   double eh, ih, ih2;
   const double *lh, *lP;                  // lambda of d_t h and of d_t Pi
   const double *P1, *P2;                  // sum_v lP_v of the first differences of Pi, the second ones of h
