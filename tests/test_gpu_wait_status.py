@@ -46,3 +46,20 @@ def test_verbs_refuse_after_a_wait_gave_up(tgh, q, N, roots):
     refuses(tgh, P.device_status)
     P.close()
     Q.close()
+
+
+def test_a_problem_starts_with_a_clean_status(tgh):
+    """The status words are lent to one problem after another: what one left behind is not the next one's."""
+    case = tgh.gauge_wave_case(eps_ko=0.5, gamma0=1.0)
+    f = tgh.gh_forest(case, 32, 1)
+    other = tgh.GHProblem(case, f, 4, margin_check=False)
+    for _ in range(3):
+        P = tgh.GHProblem(case, f, 4, margin_check=False)
+        u = P.initial_state(P.statevector(), 0.0)
+        P.max_speed(u, 0.0)
+        P.set_wait_limit(-1)
+        P.gh_rhs(torch.zeros_like(u), u, 0.0)
+        refuses(tgh, lambda: P.max_speed(u, 0.0))
+        other.max_speed(u, 0.0)
+        P.close()
+    other.close()

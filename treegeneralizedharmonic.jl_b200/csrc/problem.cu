@@ -9,6 +9,7 @@
 #include <cstring>
 #include <string>
 #include <map>
+#include <mutex>
 #include <unordered_map>
 #include <vector>
 
@@ -195,6 +196,34 @@ struct tgh_problem {
 static int fail(tgh_problem* p, int code, const std::string& msg) {
   p->err = msg;
   return code;
+}
+
+// The problems' status words. Pinned memory takes a millisecond to allocate and half of one to free, so words are lent
+// from pages of 1024 that the process keeps: one page, unless more problems than that live at once.
+static std::mutex wait_words_mutex;
+static std::vector<int*> wait_words_free;
+static cudaError_t lend_wait_word(tgh_problem* p) {
+  std::lock_guard<std::mutex> lock(wait_words_mutex);
+  if (wait_words_free.empty()) {
+    constexpr int words = 1024;
+    int* page = nullptr;
+    const cudaError_t e = cudaHostAlloc((void**)&page, words * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    for (int i = words - 1; i >= 0; --i) wait_words_free.push_back(page + i);
+  }
+  int* w = wait_words_free.back();
+  const cudaError_t e = cudaHostGetDevicePointer((void**)&p->dev_err, w, 0);
+  if (e != cudaSuccess) return e;
+  wait_words_free.pop_back();
+  p->wait_word = w;
+  *p->wait_word = 0;
+  return cudaSuccess;
+}
+static void return_wait_word(tgh_problem* p) {
+  if (!p->wait_word) return;
+  std::lock_guard<std::mutex> lock(wait_words_mutex);
+  wait_words_free.push_back(const_cast<int*>(p->wait_word));
+  p->wait_word = nullptr;
 }
 
 // whether a bounded device wait has given up since the last tgh_device_status: the state on the device is then
@@ -1230,11 +1259,7 @@ static int setup_device(tgh_problem* p) {
   CK(alloc_work(p, &p->work));
   CK(cudaMalloc(&p->scratch, 2 * sizeof(unsigned long long)));
   CK(cudaMalloc(&p->bcounts, 3 * sizeof(unsigned long long)));
-  void* word = nullptr;
-  CK(cudaHostAlloc(&word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-  p->wait_word = (volatile int*)word;
-  *p->wait_word = 0;
-  CK(cudaHostGetDevicePointer((void**)&p->dev_err, word, 0));
+  CK(lend_wait_word(p));
   CK(cudaMalloc(&p->coef, (size_t)NCOEF * p->SX * p->nb * sizeof(double)));
   p->npart = (int)grid_for(p->npts, 128);
   CK(cudaMalloc(&p->part, (3 * (size_t)p->npart + 2) * sizeof(double)));
@@ -1302,7 +1327,7 @@ void tgh_problem_destroy(tgh_problem* p) {
   for (auto* pp : p->ptpts)
     if (pp) cudaFree(pp);
   // after the cudaFrees, which wait for the device: no kernel can still write the word
-  if (p->wait_word) cudaFreeHost((void*)p->wait_word);
+  return_wait_word(p);
   delete p;
 }
 
