@@ -19,7 +19,7 @@ Workloads (seeded synthetic inputs, fully specified by their parameters):
   hierarchy           (the default) the hole of kerr_schild_static boosted to v = 0.1 along x,
                       on [-40,40]^3 refined around its path in 5 levels to 2472 blocks of 32^3
                       (finest h = 5/256), algebraic Kerr-Schild gauge source, moving :damped
-                      core; ~117 GB on the device in the batched form. The plain forms are
+                      core; ~139 GB on the device in the batched form. The plain forms are
                       timed after the batched problem is released, on a problem of their own
   kerr_schild_static  static Kerr-Schild hole M=1, a=7/10 on [-8,8]^3, 64 blocks of 32^3
                       (h = 1/8), Dirichlet faces, :damped interior r_0=0.8 r_1=1.3 rho_max=4/M,

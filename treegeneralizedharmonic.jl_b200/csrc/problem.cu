@@ -1207,8 +1207,8 @@ static int setup_host(tgh_problem* p, const tgh_config* cfg, const tgh_mesh* m, 
   if (cfg->precision != TGH_PREC_FP64 && cfg->precision != TGH_PREC_MIXED)
     return fail(p, TGH_ERR_ARG, "the precision must be TGH_PREC_FP64 or TGH_PREC_MIXED");
   p->mixed = cfg->precision == TGH_PREC_MIXED;
-  // where the TMA-staged Pi kernel applies it is the faster one at every size measured (8 blocks of 32^3: 92 us a
-  // stage against 121 through L1; 64 blocks: 661 against 840), so it is what an untuned problem runs
+  // where the TMA-staged Pi kernel applies it is the faster one at every size measured (8 blocks of 32^3: 86-99 us a
+  // stage against 105-113 through L1; 64 blocks: 520-614 against 685-746), so it is what an untuned problem runs
   if (q == 4 && m->N == 32 && !p->mixed) p->pi_variant = PI_TMA;
   if (p->intr) {
     if (!(cfg->r0 > 0.0 && cfg->r1 > cfg->r0))

@@ -17,9 +17,9 @@
 // d_y d_z h outer sums of D_z h. An inner sum is formed once, by the thread that owns the pair (those
 // beyond the tile by extra tasks), and read by the points around it from shared memory: 39 instead of 91
 // FP64 operations a point and component, and 45 instead of 68 shared loads a pair, against forming them
-// at each point. On 64 blocks a stage takes 638 us (777 us with every inner sum formed where it is used and
-// every copy of a shared point computed); it is bound by DRAM (2.8 GB, 4.4 TB/s) and by the latency of its shared
-// loads at 12 warps an SM.
+// at each point. On 64 blocks a stage takes 520 to 614 us by stage (777 us with every inner sum formed where it is
+// used and every copy of a shared point computed; 685 to 746 us the one-point kernel); it is bound by DRAM (2.35 to
+// 2.8 GB, 4.4 TB/s) and by the latency of its shared loads at 12 warps an SM.
 //
 // The arithmetic is the one-point kernel's, operation for operation (the same stencil sums in
 // the same order and the same contraction with the head's coefficients), so both kernels give
