@@ -33,7 +33,7 @@ def test_verbs_refuse_after_a_wait_gave_up(tgh, q, N, roots):
         # and so does every verb after, whatever the limit, until the status is read
         for verb in (lambda: P.gh_rhs(du, u, 0.0), lambda: P.step_batched(u.clone(), 0.0, dt, 1),
                      lambda: P.rk4_step(u.clone(), 0.0, dt), lambda: P.prepare(u, 0.0), lambda: P.error_norm(u, 0.0),
-                     lambda: P.gh_constraint(u, 0.0), lambda: P.copy_work(), lambda: P.time_rhs(u, 0.0, nlaunch=1),
+                     lambda: P.gh_constraint(u, 0.0), lambda: P.stage_limit(u, 0.0), lambda: P.copy_work(), lambda: P.time_rhs(u, 0.0, nlaunch=1),
                      lambda: Q.transfer_from(P, u, 0.0, du)):
             refuses(tgh, verb)
         refuses(tgh, P.device_status)

@@ -1099,6 +1099,7 @@ static int apply_bounds_impl(tgh_problem* p, double* u, double t, const tgh_boun
 // gh_stage_limiter! then gh_step_limiter! (src/stepping.jl:91-95): the range projection, when
 // the problem has bounds, with its accounting (src/bounds.jl:757-776); then the :pasted paste
 static int stage_limit_impl(tgh_problem* p, double* u, double t) {
+  if (int st = waits_ok(p)) return st;
   if (p->has_bounds) {
     long n = 0, nf = 0;
     double rm = 0.0;
@@ -1782,6 +1783,8 @@ static int fill_target_impl(tgh_problem* p, const double* u, double t_f, double 
   if (int s = fitted_check(p)) return s;
   if (!std::isfinite(t_f) || !(r_fill >= 0.0) || !(dt >= 0.0))
     return fail(p, TGH_ERR_ARG, "the fill needs a finite t_f, r_fill >= 0 and dt >= 0");
+  if (u)
+    if (int st = waits_ok(p)) return st;
   const int phases = (!u && dt > 0.0) ? 3 : 1;
   for (int ph = 0; ph < phases; ++ph)
     fill_target_kernel<<<grid_for(p->npts, 128), 128, 0, p->stream>>>(p->tw, u, p->blk, p->geo, p->npts, p->cs,
