@@ -21,13 +21,14 @@ def _rhs_error(tgh, oracle, case, f, q, t, precision="fp64"):
     return err
 
 
-# the interior kernel's points a CTA on 8 blocks around the hole and 148 SMs: 128 up to 11^3, 256 at 13^3, 512 from 16^3
-@pytest.mark.parametrize("N", [11, 13, 16])
+# the interior kernel's points a CTA around the hole and 148 SMs: on 8 blocks 128 up to 15^3 and 512 from 16^3 on, where
+# one block of 27 holds the sphere 128 up to 32^3 and 512 at 33^3
+@pytest.mark.parametrize("N,roots,halfwidth", [(11, 2, 2.0), (15, 2, 2.0), (16, 2, 2.0), (32, 3, 4.0), (33, 3, 4.0)])
 @pytest.mark.parametrize("variant,v", [("damped", 0.0), ("damped", 0.1), ("frozen", 0.0)])
-def test_interior_on_small_meshes(tgh, oracle, N, variant, v):
-    case = tgh.kerr_schild_case(a=0.7, v=v, halfwidth=2.0, variant=variant, gauge="algebraic")
+def test_interior_on_small_meshes(tgh, oracle, N, roots, halfwidth, variant, v):
+    case = tgh.kerr_schild_case(a=0.7, v=v, halfwidth=halfwidth, variant=variant, gauge="algebraic")
     # the bound of the right-hand side's parity everywhere
-    assert _rhs_error(tgh, oracle, case, tgh.gh_forest(case, N, 2), 4, 0.3) < 1e-12
+    assert _rhs_error(tgh, oracle, case, tgh.gh_forest(case, N, roots), 4, 0.3) < 1e-12
 
 
 # the one-point Pi kernel's registers: a block's launch is below the line (27 CTAs), the mesh's of 1,688 above it

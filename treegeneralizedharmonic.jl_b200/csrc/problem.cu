@@ -969,14 +969,14 @@ static int launch_interior(tgh_problem* p, const RhsArgs& a, int mode, cudaStrea
     L = &p->ilist;
   }
   if (L->n > 0) {
-    // Few points a CTA while the CTAs find an SM each, else many, so that the lists fill whole warps. us a right-hand
-    // side with 512 points a CTA against 128, where 128 makes 18 CTAs (one block of 12^3 holds the sphere) 119 against
-    // 105, 144 CTAs (a moving hole in 8 of 12^3) 337 against 289, 312 CTAs (8 of 16^3) 78 against 91, 2248 CTAs (8 of
-    // 32^3) 249 against 267.
+    // Few points a CTA while all of the CTAs are resident (two an SM, by their registers), else many, so that the lists
+    // fill whole warps. us a right-hand side with 512 points a CTA against 128, where 128 makes 18
+    // CTAs (one block of 12^3 holds the sphere) 119 against 105, 154 CTAs (the sphere reaches from one of 27 blocks of 13^3
+    // into six more) 148 against 124, 216 CTAs (a moving hole in 8 of 14^3) 406 against 362, 312 CTAs (8 of 16^3) 78
+    // against 83, 432 CTAs (8 of 18^3) 92 against 102, 2248 CTAs (8 of 32^3) 249 against 267.
     int chunk = 128;
     auto ctas = [&] { return (long)L->n * ((p->S + chunk - 1) / chunk); };
-    if (ctas() > p->sms) chunk = 256;
-    if (ctas() > p->sms) chunk = INTERIOR_CHUNK;
+    if (ctas() > 2 * p->sms) chunk = INTERIOR_CHUNK;
     const unsigned grid = (unsigned)ctas();
     if (mode == MODE_DU)
       interior_kernel<MODE_DU><<<grid, 128, 0, s>>>(p->cs, a, L->dev, chunk);
