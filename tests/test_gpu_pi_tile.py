@@ -97,14 +97,19 @@ def test_a_tile_wait_that_runs_out_is_reported(tgh, q, N, limit):
     u = P.initial_state(P.statevector(), 0.25)
     ref, du = torch.zeros_like(u), torch.zeros_like(u)
     P.gh_rhs(ref, u, 0.25)
-    torch.cuda.synchronize()
     P.set_wait_limit(limit)
-    start = time.perf_counter()
-    P.gh_rhs(du, u, 0.25)
-    with pytest.raises(tgh._abi.TGHError) as e:
-        P.device_status()
-    assert e.value.code == tgh._abi.TGH_ERR_TIMEOUT
-    assert time.perf_counter() - start < 0.1  # the launches take under a millisecond
+    took = []
+    for _ in range(3):
+        torch.cuda.synchronize()
+        start = time.perf_counter()
+        P.gh_rhs(du, u, 0.25)
+        with pytest.raises(tgh._abi.TGHError) as e:
+            P.device_status()
+        took.append(time.perf_counter() - start)
+        assert e.value.code == tgh._abi.TGH_ERR_TIMEOUT
+    # the launches take under a millisecond, 2^24 polls 0.4 s at the least (50 cycles each at 1.965 GHz); the quickest of
+    # three, as the host may be held up in one
+    assert min(took) < 0.2
     P.set_wait_limit(1 << 26)
     P.gh_rhs(du, u, 0.25)
     P.device_status()
